@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/qwc.h"
 
 struct qwc_hal {
@@ -54,6 +56,15 @@ inline cudaError_t qwc_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+// Lets KERNEL use `bytes` of dynamic shared memory: set once per device (racing first calls set the same value).
+template <auto KERNEL> inline int qwc_allow_smem(const qwc_hal* hal, int bytes) {
+    static std::atomic<bool> configured[64];
+    if (!configured[hal->device & 63].load(std::memory_order_acquire)) {
+        QWC_CUDA_TRY(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        configured[hal->device & 63].store(true, std::memory_order_release);
+    }
+    return QWC_OK;
+}
 #endif
 
 // Argument checks shared by the doors (qwc_api.cu): every refusal a later launch could make, without launching.
@@ -100,6 +111,52 @@ __device__ __forceinline__ float qwc_inv_sqrt32() { return __uint_as_float(0x3E3
 __device__ __forceinline__ float fwht_xor_stage(float v, int lane_mask, bool upper) {
     float o = __shfl_xor_sync(0xFFFFFFFFu, v, lane_mask);
     return upper ? __fsub_rn(o, v) : __fadd_rn(v, o);
+}
+
+// FWHT-32 of one 32-element block held by the four lanes of a quad, lane t holding elements 8 t .. 8 t + 7: three in-lane
+// butterfly stages and two xor-shuffle stages, the reference's h = 1, 2, 4, 8, 16 order, then the 1/sqrt(32) scale.  A lane
+// moves 16 or 32 bytes per access and shuffles twice per element; one lane per element moves 2 or 4 bytes and shuffles five
+// times.  fma(v, +-1, o) is the rounded sum or difference itself.
+__device__ __forceinline__ void fwht32_quad(float f[8], int t4) {
+#pragma unroll
+    for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if ((i & h) == 0) {
+                const float a = f[i], b = f[i + h];
+                f[i] = __fadd_rn(a, b);
+                f[i + h] = __fsub_rn(a, b);
+            }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+        const float sg = (t4 & m) ? -1.0f : 1.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float o = __shfl_xor_sync(0xFFFFFFFFu, f[i], m);
+            f[i] = __fmaf_rn(f[i], sg, o);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = __fmul_rn(f[i], qwc_inv_sqrt32());
+}
+// The same on eight f16 values, one rounding at the end.
+__device__ __forceinline__ uint4 fwht32_quad_f16(uint4 raw, int t4) {
+    __half2* hv = reinterpret_cast<__half2*>(&raw);
+    float f[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { f[2 * i] = __low2float(hv[i]); f[2 * i + 1] = __high2float(hv[i]); }
+    fwht32_quad(f, t4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) hv[i] = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+    return raw;
+}
+// Eight consecutive f16 values: one 16-byte load, or element loads where the rows are not 16-byte aligned.
+__device__ __forceinline__ uint4 load_f16x8(const __half* src, bool vec) {
+    if (vec) return *reinterpret_cast<const uint4*>(src);
+    __half tmp[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tmp[i] = src[i];
+    return *reinterpret_cast<const uint4*>(tmp);
 }
 
 // Programmatic dependent launch, used between the kernels of one operator chain: a kernel lets its successor be

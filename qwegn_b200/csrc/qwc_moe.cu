@@ -121,56 +121,6 @@ __global__ void __launch_bounds__(128) qwc_moe_route_kernel(const float* __restr
     }
 }
 
-// Router logits: y[t, e] = x[t, :] . W[e, :], f32 accumulate (the reference's qwg_router_gemm,
-// Sources/QWMetal/subsystems/qwrouter.metal:460-520; host door QWGemmMoERouter.swift:78-125).  The router weight is a
-// raw, un-rotated plane (bf16, f16 or f32), the activations are the plain (un-rotated) hidden states (f16 or f32).
-// A CTA computes 64 tokens x 64 experts; K goes through shared memory 32 columns at a time; a thread owns a 4 x 4
-// block (tokens 4 ty .. 4 ty + 3, experts tx, tx + 16, tx + 32, tx + 48).
-__device__ __forceinline__ float router_cvt(float v) { return v; }
-__device__ __forceinline__ float router_cvt(__half v) { return __half2float(v); }
-__device__ __forceinline__ float router_cvt(unsigned short v) { return __uint_as_float(static_cast<uint32_t>(v) << 16); }   // bf16 bits
-
-template <typename XT, typename WT>
-__global__ void __launch_bounds__(256) qwc_moe_router_gemm_kernel(const XT* __restrict__ x, int64_t ldx, const WT* __restrict__ w,
-                                                                  int t_rows, int e, int h, float* __restrict__ y) {
-    pdl_enter();
-    __shared__ float xs[64][33];
-    __shared__ float ws[64][33];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int t0 = blockIdx.y * 64, e0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < h; k0 += 32) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int r = (tid >> 5) + 8 * i, c = tid & 31;
-            xs[r][c] = t0 + r < t_rows ? router_cvt(x[static_cast<int64_t>(t0 + r) * ldx + k0 + c]) : 0.0f;
-            ws[r][c] = e0 + r < e ? router_cvt(w[static_cast<int64_t>(e0 + r) * h + k0 + c]) : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int kk = 0; kk < 32; ++kk) {
-            float xv[4], wv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                xv[i] = xs[4 * ty + i][kk];
-                wv[i] = ws[tx + 16 * i][kk];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int t = t0 + 4 * ty + i, ex = e0 + tx + 16 * j;
-            if (t < t_rows && ex < e) y[static_cast<int64_t>(t) * e + ex] = acc[i][j];
-        }
-}
-
 // Tile j of expert ex for a bank with `rows` rows per expert.  paired != 0 (gate||up bank feeding a SwiGLU epilogue):
 // the tile is 64 gate rows followed by the 64 up rows that pair with them, and its output columns are the 64 rows of h.
 __device__ __forceinline__ qwc_moe_tile moe_make_tile(int ex, int rows, int j, int paired, int x_row0, int x_rows) {
@@ -315,40 +265,8 @@ __device__ __forceinline__ void moe_gather_items(const __half* __restrict__ x, i
         const int64_t pr = static_cast<int64_t>(prq);
         const __half* src = x + static_cast<int64_t>(live ? (sorted_tok != nullptr ? sorted_tok[pr] : static_cast<int32_t>(pr)) : 0) * ldx + u * 32 + 8 * t4;
         uint4 raw = make_uint4(0, 0, 0, 0);
-        if (live) {
-            if (vec) raw = *reinterpret_cast<const uint4*>(src);
-            else {
-                __half tmp[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) tmp[i] = src[i];
-                raw = *reinterpret_cast<const uint4*>(tmp);
-            }
-        }
-        if (rotate) {
-            __half2 hv[4] = {*reinterpret_cast<__half2*>(&raw.x), *reinterpret_cast<__half2*>(&raw.y),
-                             *reinterpret_cast<__half2*>(&raw.z), *reinterpret_cast<__half2*>(&raw.w)};
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { f[2 * i] = __low2float(hv[i]); f[2 * i + 1] = __high2float(hv[i]); }
-#pragma unroll
-            for (int s = 1; s < 8; s <<= 1)
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if ((i & s) == 0) {
-                        const float a = f[i], b = f[i + s];
-                        f[i] = __fadd_rn(a, b);
-                        f[i + s] = __fsub_rn(a, b);
-                    }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = fwht_xor_stage(f[i], 1, (t4 & 1) != 0);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = fwht_xor_stage(f[i], 2, (t4 & 2) != 0);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                hv[i] = __floats2half2_rn(__fmul_rn(f[2 * i], qwc_inv_sqrt32()), __fmul_rn(f[2 * i + 1], qwc_inv_sqrt32()));
-            raw = make_uint4(*reinterpret_cast<uint32_t*>(&hv[0]), *reinterpret_cast<uint32_t*>(&hv[1]),
-                             *reinterpret_cast<uint32_t*>(&hv[2]), *reinterpret_cast<uint32_t*>(&hv[3]));
-        }
+        if (live) raw = load_f16x8(src, vec != 0);
+        if (rotate) raw = fwht32_quad_f16(raw, t4);
         if (live) *reinterpret_cast<uint4*>(xs + pr * h + u * 32 + 8 * t4) = raw;
     }
 }
@@ -736,37 +654,6 @@ int64_t qwc_moe_max_tiles(int64_t pairs, int64_t e, int64_t rows_per_expert) {
     int64_t tx = e + pairs / moe_tile_rows(pairs, e);
     if (tx > pairs) tx = pairs;
     return tx * ((rows_per_expert + kTileW - 1) / kTileW);
-}
-
-int qwc_moe_router_gemm(qwc_hal* hal, qwc_stream stream, const void* x, int32_t x_dtype, int64_t ldx, int64_t t, int64_t h,
-                        const void* w, int32_t w_dtype, int64_t e, float* logits) {
-    qwc_clear_error();
-    if (!hal) return qwc_fail(QWC_ERR_BAD_SHAPE, "hal is null");
-    // QWGemmMoERouter.swift:82: the router GEMM needs K % 32 == 0
-    if (h <= 0 || h % 32 != 0) return qwc_fail(QWC_ERR_BAD_GEOMETRY, "hidden=%lld must be a positive multiple of 32", (long long)h);
-    if (e <= 0 || t < 0) return qwc_fail(QWC_ERR_BAD_SHAPE, "bad extents");
-    if (t == 0) return QWC_OK;
-    if (ldx < h) return qwc_fail(QWC_ERR_BAD_SHAPE, "ldx < hidden");
-    if (!x || !w || !logits) return qwc_fail(QWC_ERR_BAD_SHAPE, "null buffer");
-    if (x_dtype != QWC_F16 && x_dtype != QWC_F32) return qwc_fail(QWC_ERR_BAD_SHAPE, "activations must be f16 or f32");
-    if (w_dtype != QWC_F16 && w_dtype != QWC_F32 && w_dtype != QWC_BF16) return qwc_fail(QWC_ERR_BAD_WEIGHTS, "router weights must be bf16, f16 or f32");
-    const dim3 grid(static_cast<unsigned>((e + 63) / 64), static_cast<unsigned>((t + 63) / 64));
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int ti = static_cast<int>(t), ei = static_cast<int>(e), hi = static_cast<int>(h);
-#define QWC_ROUTER_LAUNCH(XT, WT) \
-    QWC_CUDA_TRY(qwc_launch_pdl(qwc_moe_router_gemm_kernel<XT, WT>, grid, dim3(256), 0, st, static_cast<const XT*>(x), ldx, static_cast<const WT*>(w), ti, ei, hi, logits))
-    if (x_dtype == QWC_F32) {
-        if (w_dtype == QWC_F32) QWC_ROUTER_LAUNCH(float, float);
-        else if (w_dtype == QWC_F16) QWC_ROUTER_LAUNCH(float, __half);
-        else QWC_ROUTER_LAUNCH(float, unsigned short);
-    } else {
-        if (w_dtype == QWC_F32) QWC_ROUTER_LAUNCH(__half, float);
-        else if (w_dtype == QWC_F16) QWC_ROUTER_LAUNCH(__half, __half);
-        else QWC_ROUTER_LAUNCH(__half, unsigned short);
-    }
-#undef QWC_ROUTER_LAUNCH
-    QWC_CUDA_TRY(cudaGetLastError());
-    return QWC_OK;
 }
 
 int qwc_moe_route(qwc_hal* hal, qwc_stream stream, const float* logits, int64_t t, int64_t e, int64_t k, int32_t norm_topk,

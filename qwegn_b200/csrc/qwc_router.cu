@@ -1,0 +1,321 @@
+// Router logits: y[t, e] = x[t, :] . W[e, :], f32 accumulate (the reference's qwg_router_gemm,
+// Sources/QWMetal/subsystems/qwrouter.metal:460-520; host door QWGemmMoERouter.swift:78-125).  The router weight is a
+// raw, un-rotated plane (bf16, f16 or f32), the activations are the plain (un-rotated) hidden states (f16 or f32).
+//
+// Two kernels:
+//  * up to kRowsTokens tokens (and buffers that are not 16-byte aligned): one CTA per expert, the whole of K spread over
+//    its threads, so that the only chain is two or three loads and one reduction;
+//  * more tokens: tensor cores (mma.sync) straight from global memory, no shared-memory operands.  A router plane is 1 MB
+//    and its contraction a thousandth of the expert GEMMs', so what counts is latency: K is split over the warps of a CTA.
+#include "qwc_common.cuh"
+
+namespace {
+
+constexpr int kRowsTokens = 8;   // tokens one pass of the row kernel serves
+// The row kernel reads x once per expert: its time grows by ~3 us per 8 tokens while the tensor-core form starts at ~8 us.
+constexpr int kRowsMaxTokens = 16;
+
+// Eight consecutive elements as f32.
+template <bool VEC> __device__ __forceinline__ void load8(const float* p, float f[8]) {
+    if (VEC) {
+        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = p[i];
+    }
+}
+template <bool VEC> __device__ __forceinline__ void load8(const __half* p, float f[8]) {
+    if (VEC) {
+        const uint4 r = *reinterpret_cast<const uint4*>(p);
+        const __half2* h = reinterpret_cast<const __half2*>(&r);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { f[2 * i] = __low2float(h[i]); f[2 * i + 1] = __high2float(h[i]); }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = __half2float(p[i]);
+    }
+}
+template <bool VEC> __device__ __forceinline__ void load8(const unsigned short* p, float f[8]) {   // bf16 bits
+    if (VEC) {
+        const uint4 r = *reinterpret_cast<const uint4*>(p);
+        const uint32_t* u = reinterpret_cast<const uint32_t*>(&r);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { f[2 * i] = __uint_as_float(u[i] << 16); f[2 * i + 1] = __uint_as_float(u[i] & 0xFFFF0000u); }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(static_cast<uint32_t>(p[i]) << 16);
+    }
+}
+
+// One expert per CTA, up to kRowsTokens tokens per blockIdx.y.  Thread i takes the 8-element chunks i, i + 128, ... of K;
+// partial sums meet by shuffles, then across the four warps in a fixed order.
+template <typename XT, typename WT, bool VEC>
+__global__ void __launch_bounds__(128) qwc_router_rows_kernel(const XT* __restrict__ x, int64_t ldx, const WT* __restrict__ w,
+                                                              int t_rows, int e, int h, float* __restrict__ y) {
+    pdl_enter();
+    __shared__ float part[4][kRowsTokens];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ex = blockIdx.x, t0 = blockIdx.y * kRowsTokens;
+    const int tn = min(kRowsTokens, t_rows - t0);
+    const WT* wr = w + static_cast<int64_t>(ex) * h;
+    const XT* xr = x + static_cast<int64_t>(t0) * ldx;
+    float acc[kRowsTokens] = {};
+    for (int c = tid * 8; c < h; c += 128 * 8) {
+        float wv[8];
+        load8<VEC>(wr + c, wv);
+#pragma unroll
+        for (int i = 0; i < kRowsTokens; ++i) {
+            if (i < tn) {
+                float xv[8];
+                load8<VEC>(xr + i * ldx + c, xv);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i] = fmaf(xv[j], wv[j], acc[i]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kRowsTokens; ++i) {
+        if (i >= tn) break;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xFFFFFFFFu, acc[i], o);
+        if (lane == 0) part[warp][i] = acc[i];
+    }
+    __syncthreads();
+    if (tid < tn) y[static_cast<int64_t>(t0 + tid) * e + ex] = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+}
+
+// ---- tensor-core form -------------------------------------------------------------------------------------------
+// An f32 product needs the operands exact: bf16 is taken as it is, f16 (11 significant bits) is the sum of two bf16 and
+// f32 (24 bits) of three, by truncation, so every plane is exact and the f32 accumulator sees the products of the f32
+// operands; only the plane pair below 2^-32 of the product is left out.  f16 x f16 needs no split (one f16 MMA).
+template <typename T> struct RouterPlanes;
+template <> struct RouterPlanes<unsigned short> { static constexpr int kPlanes = 1, kRaw = 4; };
+template <> struct RouterPlanes<__half> { static constexpr int kPlanes = 2, kRaw = 4; };
+template <> struct RouterPlanes<float> { static constexpr int kPlanes = 3, kRaw = 8; };
+
+// 8 elements: raw words -> planes of 4 words (pairs of bf16 in element order).
+__device__ __forceinline__ void split_planes(const uint32_t* raw, uint32_t (*pl)[4], const unsigned short*) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pl[0][i] = raw[i];
+}
+__device__ __forceinline__ uint32_t f16x2_to_bf16x2(uint32_t v) {   // exact for values of at most 8 significant bits
+    const __half2 h = *reinterpret_cast<const __half2*>(&v);
+    return __byte_perm(__float_as_uint(__low2float(h)), __float_as_uint(__high2float(h)), 0x7632);
+}
+__device__ __forceinline__ void split_planes(const uint32_t* raw, uint32_t (*pl)[4], const __half*) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t hi = raw[i] & 0xFFF8FFF8u;   // the upper 8 significant bits
+        const __half2 x = *reinterpret_cast<const __half2*>(&raw[i]), h2 = *reinterpret_cast<const __half2*>(&hi);
+        const __half2 lo2 = __hsub2(x, h2);         // exact: the lower 3 bits
+        // infinities and NaNs travel in the first plane alone (inf - inf would make a NaN of an infinity)
+        const uint32_t fin = __hle2_mask(__habs2(x), __floats2half2_rn(65504.0f, 65504.0f));
+        pl[0][i] = f16x2_to_bf16x2(hi | (raw[i] & ~fin));
+        pl[1][i] = f16x2_to_bf16x2(*reinterpret_cast<const uint32_t*>(&lo2) & fin);
+    }
+}
+__device__ __forceinline__ void split_planes(const uint32_t* raw, uint32_t (*pl)[4], const float*) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float a = __uint_as_float(raw[2 * i]), b = __uint_as_float(raw[2 * i + 1]);
+        const bool fa = fabsf(a) <= 3.402823466e38f, fb = fabsf(b) <= 3.402823466e38f;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+            if (p == 0) {   // a NaN must not lose its low payload bits and turn into an infinity
+                if (a != a) ua |= 0x00400000u;
+                if (b != b) ub |= 0x00400000u;
+            }
+            pl[p][i] = __byte_perm(ua, ub, 0x7632);
+            a = fa ? __fsub_rn(a, __uint_as_float(ua & 0xFFFF0000u)) : 0.0f;
+            b = fb ? __fsub_rn(b, __uint_as_float(ub & 0xFFFF0000u)) : 0.0f;
+        }
+    }
+}
+
+template <bool F16>
+__device__ __forceinline__ void router_mma(float d[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if (F16)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int RAW, typename T> __device__ __forceinline__ void load_raw(const T* p, uint32_t* r) {
+    const uint4 a = *reinterpret_cast<const uint4*>(p);
+    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+    if (RAW == 8) {
+        const uint4 b = reinterpret_cast<const uint4*>(p)[1];
+        r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+    }
+}
+
+// A warp owns 32 tokens x 32 experts of the CTA's (32 MW) x (32 NW) tile and every KW-th 32-wide step of K.  Lane t of a
+// quad reads the 8 consecutive k [8 t, 8 t + 8) of a step for its rows, one 16-byte load (two for f32) per row: the two
+// MMAs of a step then take k slots in that permuted order, the same for both operands, so nothing is shuffled or staged.
+// The next step's words are fetched before this step's are used.  The KW partial tiles meet in shared memory and are
+// summed in a fixed order.
+template <typename XT, typename WT, int MW, int NW, int KW>
+__global__ void __launch_bounds__(MW * NW * KW * 32, 1) qwc_router_mma_kernel(const XT* __restrict__ x, int64_t ldx, const WT* __restrict__ w,
+                                                                             int t_rows, int e, int h, float* __restrict__ y) {
+    constexpr bool kF16 = sizeof(XT) == 2 && RouterPlanes<WT>::kPlanes == 2;   // x f16 (2-byte x is always f16), w f16
+    constexpr int PX = kF16 ? 1 : RouterPlanes<XT>::kPlanes, PW = kF16 ? 1 : RouterPlanes<WT>::kPlanes;
+    constexpr int RX = RouterPlanes<XT>::kRaw, RW = RouterPlanes<WT>::kRaw;
+    constexpr int TM = 32 * MW, TN = 32 * NW;
+    extern __shared__ float4 part[];   // [KW][warps of a K slice][8 fragments][32 lanes]
+    pdl_enter();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gid = lane >> 2, t4 = lane & 3;
+    const int kw = warp % KW, pos = warp / KW, mw = pos % MW, nw = pos / MW;
+    const int t0 = blockIdx.y * TM + mw * 32, e0 = blockIdx.x * TN + nw * 32;
+    // rows past the end read the last row again; their results are not stored
+    const XT* xp[4];
+    const WT* wp[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        xp[i] = x + static_cast<int64_t>(min(t0 + 8 * i + gid, t_rows - 1)) * ldx + 8 * t4;
+        wp[i] = w + static_cast<int64_t>(min(e0 + 8 * i + gid, e - 1)) * h + 8 * t4;
+    }
+    float d[2][4][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) d[i][j][q] = 0.0f;
+    const int steps = h / 32;
+    uint32_t xr[4][RX], wr[4][RW];
+    if (kw < steps) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            load_raw<RX>(xp[i] + kw * 32, xr[i]);
+            load_raw<RW>(wp[i] + kw * 32, wr[i]);
+        }
+    }
+    for (int s = kw; s < steps; s += KW) {
+        uint32_t xpl[4][PX][4], wpl[4][PW][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (kF16) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { xpl[i][0][j] = xr[i][j]; wpl[i][0][j] = wr[i][j]; }
+            } else {
+                split_planes(xr[i], xpl[i], static_cast<const XT*>(nullptr));
+                split_planes(wr[i], wpl[i], static_cast<const WT*>(nullptr));
+            }
+        }
+        if (s + KW < steps) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                load_raw<RX>(xp[i] + (s + KW) * 32, xr[i]);
+                load_raw<RW>(wp[i] + (s + KW) * 32, wr[i]);
+            }
+        }
+        // smallest plane pairs first
+#pragma unroll
+        for (int lvl = PX + PW - 2; lvl >= 0; --lvl) {
+            if (lvl > 3) continue;
+#pragma unroll
+            for (int a = 0; a < PX; ++a) {
+                const int b = lvl - a;
+                if (b < 0 || b >= PW) continue;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int q = 0; q < 2; ++q)
+                            router_mma<kF16>(d[i][j], xpl[2 * i][a][2 * q], xpl[2 * i + 1][a][2 * q], xpl[2 * i][a][2 * q + 1],
+                                             xpl[2 * i + 1][a][2 * q + 1], wpl[j][b][2 * q], wpl[j][b][2 * q + 1]);
+            }
+        }
+    }
+    constexpr int kPos = MW * NW;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            part[((kw * kPos + pos) * 8 + i * 4 + j) * 32 + lane] = make_float4(d[i][j][0], d[i][j][1], d[i][j][2], d[i][j][3]);
+    __syncthreads();
+    // the KW warps of a position share its eight fragments
+    for (int f = kw; f < 8; f += KW) {
+        float4 s = part[(pos * 8 + f) * 32 + lane];
+#pragma unroll
+        for (int k = 1; k < KW; ++k) {
+            const float4 v = part[((k * kPos + pos) * 8 + f) * 32 + lane];
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        const int i = f >> 2, j = f & 3;
+        const float v4[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int t = t0 + 16 * i + gid + 8 * (q >> 1), ex = e0 + 8 * j + 2 * t4 + (q & 1);
+            if (t < t_rows && ex < e) y[static_cast<int64_t>(t) * e + ex] = v4[q];
+        }
+    }
+}
+
+template <typename XT, typename WT, int MW, int NW, int KW>
+int launch_router_mma(const qwc_hal* hal, cudaStream_t st, const void* x, int64_t ldx, const void* w, int t, int e, int h, float* y) {
+    constexpr int kSmem = KW * MW * NW * 8 * 32 * 16;
+    if (kSmem > 48 * 1024)
+        if (int rc = qwc_allow_smem<qwc_router_mma_kernel<XT, WT, MW, NW, KW>>(hal, kSmem)) return rc;
+    const dim3 grid(static_cast<unsigned>((e + 32 * NW - 1) / (32 * NW)), static_cast<unsigned>((t + 32 * MW - 1) / (32 * MW)));
+    QWC_CUDA_TRY(qwc_launch_pdl(qwc_router_mma_kernel<XT, WT, MW, NW, KW>, grid, dim3(MW * NW * KW * 32), kSmem, st,
+                                static_cast<const XT*>(x), ldx, static_cast<const WT*>(w), t, e, h, y));
+    return QWC_OK;
+}
+
+template <typename XT, typename WT>
+int launch_router(const qwc_hal* hal, cudaStream_t st, const void* x, int64_t ldx, const void* w, int t, int e, int h, float* y) {
+    const bool vec = (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16 == 0 && ldx % (16 / static_cast<int>(sizeof(XT))) == 0;
+    if (t <= kRowsMaxTokens || !vec) {
+        const dim3 grid(static_cast<unsigned>(e), static_cast<unsigned>((t + kRowsTokens - 1) / kRowsTokens));
+        const XT* xp = static_cast<const XT*>(x);
+        const WT* wp = static_cast<const WT*>(w);
+        if (vec) QWC_CUDA_TRY(qwc_launch_pdl(qwc_router_rows_kernel<XT, WT, true>, grid, dim3(128), 0, st, xp, ldx, wp, t, e, h, y));
+        else QWC_CUDA_TRY(qwc_launch_pdl(qwc_router_rows_kernel<XT, WT, false>, grid, dim3(128), 0, st, xp, ldx, wp, t, e, h, y));
+        return QWC_OK;
+    }
+    // f32 operands hold three planes each in registers: half the warps, twice the registers
+    constexpr int kHalf = sizeof(XT) == 4 || sizeof(WT) == 4 ? 2 : 1;
+    if (t <= 64) return launch_router_mma<XT, WT, 1, 1, 16 / kHalf>(hal, st, x, ldx, w, t, e, h, y);
+    return launch_router_mma<XT, WT, 2, 2, 4 / kHalf>(hal, st, x, ldx, w, t, e, h, y);
+}
+
+}  // namespace
+
+extern "C" int qwc_moe_router_gemm(qwc_hal* hal, qwc_stream stream, const void* x, int32_t x_dtype, int64_t ldx, int64_t t, int64_t h,
+                                   const void* w, int32_t w_dtype, int64_t e, float* logits) {
+    qwc_clear_error();
+    if (!hal) return qwc_fail(QWC_ERR_BAD_SHAPE, "hal is null");
+    // QWGemmMoERouter.swift:82: the router GEMM needs K % 32 == 0
+    if (h <= 0 || h % 32 != 0) return qwc_fail(QWC_ERR_BAD_GEOMETRY, "hidden=%lld must be a positive multiple of 32", (long long)h);
+    if (e <= 0 || t < 0) return qwc_fail(QWC_ERR_BAD_SHAPE, "bad extents");
+    if (t == 0) return QWC_OK;
+    if (ldx < h) return qwc_fail(QWC_ERR_BAD_SHAPE, "ldx < hidden");
+    if (!x || !w || !logits) return qwc_fail(QWC_ERR_BAD_SHAPE, "null buffer");
+    if (x_dtype != QWC_F16 && x_dtype != QWC_F32) return qwc_fail(QWC_ERR_BAD_SHAPE, "activations must be f16 or f32");
+    if (w_dtype != QWC_F16 && w_dtype != QWC_F32 && w_dtype != QWC_BF16) return qwc_fail(QWC_ERR_BAD_WEIGHTS, "router weights must be bf16, f16 or f32");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // grid.y carries the tokens: at most 65535 blocks of 8 in one launch
+    for (int64_t t0 = 0; t0 < t; t0 += 262144) {
+        const int ti = static_cast<int>(t - t0 < 262144 ? t - t0 : 262144), ei = static_cast<int>(e), hi = static_cast<int>(h);
+        const char* xp = static_cast<const char*>(x) + t0 * ldx * (x_dtype == QWC_F32 ? 4 : 2);
+        float* yp = logits + t0 * e;
+        int rc;
+        if (x_dtype == QWC_F32) {
+            rc = w_dtype == QWC_F32   ? launch_router<float, float>(hal, st, xp, ldx, w, ti, ei, hi, yp)
+                 : w_dtype == QWC_F16 ? launch_router<float, __half>(hal, st, xp, ldx, w, ti, ei, hi, yp)
+                                      : launch_router<float, unsigned short>(hal, st, xp, ldx, w, ti, ei, hi, yp);
+        } else {
+            rc = w_dtype == QWC_F32   ? launch_router<__half, float>(hal, st, xp, ldx, w, ti, ei, hi, yp)
+                 : w_dtype == QWC_F16 ? launch_router<__half, __half>(hal, st, xp, ldx, w, ti, ei, hi, yp)
+                                      : launch_router<__half, unsigned short>(hal, st, xp, ldx, w, ti, ei, hi, yp);
+        }
+        if (rc) return rc;
+    }
+    return QWC_OK;
+}

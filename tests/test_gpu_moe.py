@@ -55,6 +55,26 @@ def test_router_gemm_matches_the_oracle(hal, oracle, t, e, h, wdt, xdt):
     assert err.value.case == "badGeometry"
 
 
+# The edges of the router's two kernels: 16 | 17 tokens between them, 64 | 65 between the tensor-core tilings, fewer K steps than
+# K-slicing warps (h = 32), ragged experts, and rows that are not 16-byte aligned (x one element in).  Bound: the operands are
+# split exactly, so only the f32 accumulation of h <= 1056 terms differs from the f64 oracle (as above).
+@pytest.mark.parametrize("t,e,h,shift", [(16, 33, 32, 0), (17, 33, 32, 0), (64, 31, 96, 0), (65, 65, 1056, 0), (129, 40, 544, 0),
+                                         (17, 8, 64, 1), (9, 8, 64, 3)])
+@pytest.mark.parametrize("xdt,wdt", [(torch.float16, torch.bfloat16), (torch.float16, torch.float16), (torch.float32, torch.float32),
+                                     (torch.float32, torch.bfloat16), (torch.float16, torch.float32)])
+def test_router_gemm_edges(hal, oracle, t, e, h, shift, xdt, wdt):
+    import qwegn_b200 as q
+    rng = np.random.default_rng(t + e + h)
+    w = torch.from_numpy(rng.normal(0.0, 0.05, (e, h)).astype(np.float32)).to(wdt).cuda()
+    x = torch.from_numpy(rng.standard_normal((t, h + shift)).astype(np.float32)).to(xdt).cuda()[:, shift:]
+    y = torch.full((t + 1, e), 7.0, dtype=torch.float32, device="cuda")
+    q.QWGemmMoE.encodeFnRouterGemm(hal, w, x, y[:t])
+    ref = oracle.router_gemm(x.float().cpu().numpy(), w.float().cpu().numpy())
+    got = y.cpu().numpy()
+    assert np.abs(got[:t] - ref).max() <= 2e-5 * np.abs(ref).max() + 1e-6
+    assert (got[t] == 7.0).all()      # nothing is written past the last token
+
+
 def test_route_refusals(hal):
     import qwegn_b200 as q
     lg = torch.zeros((2, 600), dtype=torch.float32, device="cuda")
