@@ -7,186 +7,286 @@
 
 namespace {
 
-// One warp decodes one 32-element unit; lane = element index inside the unit.
-template <int FMT>
-__device__ __forceinline__ float decode_element(const uint8_t* __restrict__ row, int64_t unit, int lane) {
-    using T = FmtTraits<FMT>;
-    const uint8_t* blk = row + (unit / T::kUnitsPerBlock) * T::kBlockBytes;
-    const uint32_t hdr = *reinterpret_cast<const uint32_t*>(blk);
-    const float s = __half2float(__ushort_as_half(static_cast<unsigned short>(hdr & 0xFFFFu)));
-    const float b = __half2float(__ushort_as_half(static_cast<unsigned short>(hdr >> 16)));
+// Both directions are bound by HBM (17408 x 5120 HQ4_G32: 56 MB of blocks against 178 MB of f16 or 356 MB of f32).  A
+// thread owns a chunk of 8 consecutive elements of the plane: with rows of whole blocks laid end to end, chunk c lives in
+// block c / (group / 8), so there is no row arithmetic; its packed bytes are one 32-bit word (two for 8-bit codes) and its
+// elements one or two 16-byte accesses.  A quad of lanes holds a 32-element unit for the rotation.  kUnroll chunks per
+// thread are loaded before the first is used.  Measured against one lane per element (5 shuffles per rotation, 2-byte
+// stores, 64-bit divisions per unit) at that size: see launch_dequant / launch_quantize.
+constexpr int kUnroll = 4;
+
+template <int FMT> struct ChunkGeom {
+    static constexpr int kChunksPerBlock = FmtTraits<FMT>::kGroup / 8;
+    static constexpr int kWords = FMT == FMT_HQ8_G32 ? 2 : 1;
+};
+
+// The chunk's header and payload words.
+template <int FMT> __device__ __forceinline__ void load_chunk(const uint8_t* __restrict__ blocks, int64_t c, uint32_t w[3]) {
+    constexpr int kPer = ChunkGeom<FMT>::kChunksPerBlock;
+    const uint32_t* blk = reinterpret_cast<const uint32_t*>(blocks + (c / kPer) * FmtTraits<FMT>::kBlockBytes);
+    const int sub = static_cast<int>(c % kPer);
+    w[0] = blk[0];
+    w[1] = blk[1 + sub * ChunkGeom<FMT>::kWords];
+    if (ChunkGeom<FMT>::kWords == 2) w[2] = blk[2 + sub * 2];
+}
+
+// q as f32 from byte `i` of v, exact.
+__device__ __forceinline__ float byte_f32(uint32_t v, int i) {
+    return __fsub_rn(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7540u + i)), 8388608.0f);
+}
+
+// fma(q, s, b) equals the reference's rounded product plus rounded sum: the product of an 11-bit scale and an at most
+// 11-bit integer is exact in f32.
+template <int FMT> __device__ __forceinline__ void decode_chunk(const uint32_t w[3], float f[8]) {
+    const float s = __half2float(__ushort_as_half(static_cast<unsigned short>(w[0] & 0xFFFFu)));
+    const float b = __half2float(__ushort_as_half(static_cast<unsigned short>(w[0] >> 16)));
     if (FMT == FMT_HQ4_G32_M5) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(blk + 4 + 4 * (lane >> 3));
-        const int j = lane & 7;
-        const uint32_t q = (w >> (4 * (j >> 1) + 16 * (j & 1))) & 0xFu;
-        return __fadd_rn(__fmul_rn(static_cast<float>(q) + 1024.0f, s), b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {   // nibbles at bits 4 i (even element) and 16 + 4 i (odd): the f16 pair (1024 + q, 1024 + q')
+            const uint32_t p = ((w[1] >> (4 * i)) & 0x000F000Fu) | 0x64006400u;
+            const __half2 h = *reinterpret_cast<const __half2*>(&p);
+            f[2 * i] = __fmaf_rn(__low2float(h), s, b);
+            f[2 * i + 1] = __fmaf_rn(__high2float(h), s, b);
+        }
     } else if (FMT == FMT_HQ8_G32) {
-        const uint32_t q = blk[4 + lane];
-        return __fadd_rn(__fmul_rn(static_cast<float>(q), s), b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = __fmaf_rn(byte_f32(w[1 + (i >> 2)], i & 3), s, b);
     } else {
-        const int e = static_cast<int>(unit % T::kUnitsPerBlock) * 32 + lane;
-        const uint32_t q = (blk[4 + (e >> 1)] >> (4 * (e & 1))) & 0xFu;
-        return __fadd_rn(__fmul_rn(static_cast<float>(q), s), b);
+        const uint32_t lo = w[1] & 0x0F0F0F0Fu, hi = (w[1] >> 4) & 0x0F0F0F0Fu;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = __fmaf_rn(byte_f32((i & 1) ? hi : lo, i >> 1), s, b);
     }
 }
 
-template <int FMT, typename OutT>
-__global__ void __launch_bounds__(256) qwc_dequant_kernel(const uint8_t* __restrict__ blocks, int64_t n, int64_t k,
-                                                          OutT* __restrict__ out, int standard_domain) {
-    using T = FmtTraits<FMT>;
-    const int lane = threadIdx.x & 31;
-    const int64_t units_per_row = k / 32;
-    const int64_t row_bytes = (k / T::kGroup) * T::kBlockBytes;
-    const int64_t total = n * units_per_row;
-    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t u = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); u < total; u += warps) {
-        const int64_t r = u / units_per_row, unit = u % units_per_row;
-        float v = decode_element<FMT>(blocks + r * row_bytes, unit, lane);
-        if (standard_domain) {
+template <typename OutT, bool VEC> __device__ __forceinline__ void store_chunk(OutT* __restrict__ out, int64_t c, const float f[8]) {
+    if constexpr (!VEC) {
 #pragma unroll
-            for (int h = 1; h < 32; h <<= 1) v = fwht_xor_stage(v, h, (lane & h) != 0);
-            v = __fmul_rn(v, qwc_inv_sqrt32());
+        for (int i = 0; i < 8; ++i) {
+            if constexpr (sizeof(OutT) == 4) out[c * 8 + i] = f[i];
+            else out[c * 8 + i] = __float2half_rn(f[i]);
         }
-        if (sizeof(OutT) == 4) reinterpret_cast<float*>(out)[r * k + unit * 32 + lane] = v;
-        else reinterpret_cast<__half*>(out)[r * k + unit * 32 + lane] = __float2half_rn(v);
+    } else if constexpr (sizeof(OutT) == 4) {
+        reinterpret_cast<float4*>(out)[2 * c] = make_float4(f[0], f[1], f[2], f[3]);
+        reinterpret_cast<float4*>(out)[2 * c + 1] = make_float4(f[4], f[5], f[6], f[7]);
+    } else {
+        uint4 o;
+        __half2* h = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+        reinterpret_cast<uint4*>(out)[c] = o;
+    }
+}
+
+template <int FMT, typename OutT, bool VEC>
+__global__ void __launch_bounds__(256) qwc_dequant_kernel(const uint8_t* __restrict__ blocks, int64_t chunks, OutT* __restrict__ out,
+                                                          int standard_domain) {
+    const int t4 = threadIdx.x & 3;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * 256;
+    // whole quads run or leave together: chunks is a multiple of 4
+    for (int64_t c0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; c0 - (threadIdx.x & 31) < chunks; c0 += kUnroll * step) {
+        uint32_t w[kUnroll][3];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u)
+            if (c0 + u * step < chunks) load_chunk<FMT>(blocks, c0 + u * step, w[u]);
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            float f[8] = {};
+            const bool live = c0 + u * step < chunks;
+            if (live) decode_chunk<FMT>(w[u], f);
+            if (standard_domain) fwht32_quad(f, t4);
+            if (live) store_chunk<OutT, VEC>(out, c0 + u * step, f);
+        }
     }
 }
 
 // In-place f16 FWHT-32: f32 butterflies, one rounding back to f16
-// (reference kernel qwg_fwht32_f16, Sources/QWMetal/gemm/qwgemm.metal:27-32).
-__global__ void __launch_bounds__(256) qwc_fwht32_f16_kernel(__half* __restrict__ x, int64_t count) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t b = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); b < count / 32; b += warps) {
-        float v = __half2float(x[b * 32 + lane]);
+// (reference kernel qwg_fwht32_f16, Sources/QWMetal/gemm/qwgemm.metal:27-32).  Eight elements per thread, `vec`: 16-byte
+// aligned x.
+__global__ void __launch_bounds__(256) qwc_fwht32_f16_kernel(__half* __restrict__ x, int64_t chunks, bool vec) {
+    pdl_enter();
+    const int t4 = threadIdx.x & 3;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * 256;
+    for (int64_t c = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; c - (threadIdx.x & 31) < chunks; c += step) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (c < chunks) v = load_f16x8(x + c * 8, vec);
+        v = fwht32_quad_f16(v, t4);
+        if (c >= chunks) continue;
+        if (vec) {
+            reinterpret_cast<uint4*>(x)[c] = v;
+        } else {
+            const __half* h = reinterpret_cast<const __half*>(&v);
 #pragma unroll
-        for (int h = 1; h < 32; h <<= 1) v = fwht_xor_stage(v, h, (lane & h) != 0);
-        x[b * 32 + lane] = __float2half_rn(__fmul_rn(v, qwc_inv_sqrt32()));
+            for (int i = 0; i < 8; ++i) x[c * 8 + i] = h[i];
+        }
     }
 }
 
 // ---- load-time quantizer -----------------------------------------------------------------------------------
 // Device twin of the reference's packers (Scripts/quantize/hq4.py:54-123, hq_blocks.py:436-517; Metal twin
 // Sources/QWMetal/quant/qw_online_quant.metal:17-55): same f32 operations in the same order, so the bytes equal
-// the Python packer's.  One warp per group; a 64-wide group is two FWHT-32 units held as two values per lane.
-__device__ __forceinline__ float warp_max(float v) {
+// the Python packer's.  The lanes of one group (a quad, eight lanes for the 64-wide groups) share its extrema by shuffles
+// and each writes the packed word of its own chunk.
+// Codes of a chunk without the division: a = (v - eb) * rcp(es) differs from the correctly rounded quotient by at most
+// 2^-22 |a| (rcp: 1 ulp = 2^-23, the product and the quotient: 2^-24 each), so unless a lies closer than that to a point where
+// the rounded quotient changes its code (half way between two integers), round(a - base) clamped to [0, top] IS the code.
+// `far` returns the largest distance of an a from the integer it rounded to; the caller divides when it is too near 1/2 (12 %
+// of the warps).  The rounding is an addition of 1.5 * 2^23: float-to-integer conversions and eight divisions per thread kept
+// the kernel at 139 us for 17408 x 5120 HQ4_G32 (63 us of traffic).  q holds the code in its low bits; NaN gives code 0.
+constexpr float kCodeErr = 2.4e-7f;   // > 2^-22
+__device__ __forceinline__ void codes_fast(const float v[8], float eb, float es, float base, float top, uint32_t q[8], float& far) {
+    const float magic = 12582912.0f, c = magic - base, r = __fdividef(1.0f, es);
+    far = 0.0f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
-__device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
-__device__ __forceinline__ float rotate32(float v, int lane) {
-#pragma unroll
-    for (int h = 1; h < 32; h <<= 1) v = fwht_xor_stage(v, h, (lane & h) != 0);
-    return __fmul_rn(v, qwc_inv_sqrt32());
+    for (int j = 0; j < 8; ++j) {
+        const float a = __fmul_rn(__fsub_rn(v[j], eb), r);
+        const float u = __fadd_rn(a, c);
+        far = fmaxf(far, fabsf(__fsub_rn(a, __fsub_rn(u, c))));
+        q[j] = __float_as_uint(fminf(fmaxf(u, magic), magic + top));
+    }
 }
 
-template <int FMT>
-__global__ void __launch_bounds__(256) qwc_quantize_kernel(const float* __restrict__ w, int64_t n, int64_t k,
-                                                           uint8_t* __restrict__ blocks, int32_t* status) {
-    using T = FmtTraits<FMT>;
-    const int lane = threadIdx.x & 31;
-    const int64_t groups_per_row = k / T::kGroup;
-    const int64_t total = n * groups_per_row;
-    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t g = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); g < total; g += warps) {
-        const float* src = w + g * T::kGroup;  // groups are contiguous in a row-major [n, k] tensor
-        uint8_t* blk = blocks + g * T::kBlockBytes;
-        float v[T::kUnitsPerBlock];
-        bool finite = true;
+template <int FMT> __device__ __forceinline__ void quantize_chunk(float v[8], int lane, int64_t c, uint8_t* __restrict__ blocks, bool live) {
+    constexpr int kPer = ChunkGeom<FMT>::kChunksPerBlock;
+    fwht32_quad(v, lane & 3);
+    uint32_t hdr, word[2] = {0u, 0u}, q[8];
+    if (FMT == FMT_HQ4_G32_M5) {
+        float amax = fabsf(v[0]);
 #pragma unroll
-        for (int u = 0; u < T::kUnitsPerBlock; ++u) {
-            const float raw = src[32 * u + lane];
-            finite = finite && isfinite(raw);
-            v[u] = rotate32(raw, lane);
+        for (int i = 1; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+        for (int o = 1; o < kPer; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+        float sc = __fdiv_rn(amax, 7.5f);
+        if (!(sc < 63.46875f)) sc = 63.46875f;
+        const __half sh = __float2half_rn(sc);
+        const float es = __half2float(sh);
+        const __half bh = __float2half_rn(__fmul_rn(-1032.0f, es));
+        const float eb = __half2float(bh);
+        const float safe = es > 0.0f ? es : 1.0f;
+        // floor(d - 1023.5) = round(d - 1024) away from a tie; d is about 1024..1039, anything else is clamped either way
+        float far;
+        codes_fast(v, eb, safe, 1024.0f, 15.0f, q, far);
+        if (far > 0.5f - 1088.0f * kCodeErr) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                q[j] = static_cast<uint32_t>(fminf(fmaxf(floorf(__fsub_rn(__fdiv_rn(__fsub_rn(v[j], eb), safe), 1023.5f)), 0.0f), 15.0f));
         }
-        if (!__all_sync(0xFFFFFFFFu, finite) && lane == 0) atomicCAS(status, 0, QWC_DEV_NONFINITE_WEIGHT);
-        if (FMT == FMT_HQ4_G32_M5) {
-            const float amax = warp_max(fabsf(v[0]));
-            float sc = __fdiv_rn(amax, 7.5f);
-            if (!(sc < 63.46875f)) sc = 63.46875f;
-            const __half sh = __float2half_rn(sc);
-            const float es = __half2float(sh);
-            const __half bh = __float2half_rn(__fmul_rn(-1032.0f, es));
-            const float eb = __half2float(bh);
-            const float safe = es > 0.0f ? es : 1.0f;
-            float qf = floorf(__fsub_rn(__fdiv_rn(__fsub_rn(v[0], eb), safe), 1023.5f));
-            qf = fminf(fmaxf(qf, 0.0f), 15.0f);
-            const uint32_t q = es > 0.0f ? static_cast<uint32_t>(qf) : 8u;
-            const int j = lane & 7;
-            uint32_t word = q << (4 * (j >> 1) + 16 * (j & 1));
-            word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1);
-            word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2);
-            word |= __shfl_xor_sync(0xFFFFFFFFu, word, 4);
-            if (j == 0) *reinterpret_cast<uint32_t*>(blk + 4 + 4 * (lane >> 3)) = word;
-            if (lane == 0)
-                *reinterpret_cast<uint32_t*>(blk) = static_cast<uint32_t>(__half_as_ushort(sh)) |
-                                                    (static_cast<uint32_t>(__half_as_ushort(bh)) << 16);
-        } else {
-            float mn = v[0], mx = v[0];
 #pragma unroll
-            for (int u = 1; u < T::kUnitsPerBlock; ++u) { mn = fminf(mn, v[u]); mx = fmaxf(mx, v[u]); }
-            mn = warp_min(mn);
-            mx = warp_max(mx);
-            const float qmax = FMT == FMT_HQ8_G32 ? 255.0f : 15.0f;
-            const __half sh = __float2half_rn(__fdiv_rn(__fsub_rn(mx, mn), qmax));
-            const __half bh = __float2half_rn(mn);
-            const float es = __half2float(sh), eb = __half2float(bh);
-            const float safe = es > 0.0f ? es : 1.0f;
-            uint32_t q[T::kUnitsPerBlock];
+        for (int j = 0; j < 8; ++j) word[0] |= (q[j] & 15u) << (4 * (j >> 1) + 16 * (j & 1));
+        if (!(es > 0.0f)) word[0] = 0x88888888u;
+        hdr = static_cast<uint32_t>(__half_as_ushort(sh)) | (static_cast<uint32_t>(__half_as_ushort(bh)) << 16);
+    } else {
+        float mn = v[0], mx = v[0];
 #pragma unroll
-            for (int u = 0; u < T::kUnitsPerBlock; ++u) {
-                float qf = rintf(__fdiv_rn(__fsub_rn(v[u], eb), safe));
-                qf = fminf(fmaxf(qf, 0.0f), qmax);
-                q[u] = es > 0.0f ? static_cast<uint32_t>(qf) : 0u;
-            }
-            if (FMT == FMT_HQ8_G32) {
-                blk[4 + lane] = static_cast<uint8_t>(q[0]);
+        for (int i = 1; i < 8; ++i) { mn = fminf(mn, v[i]); mx = fmaxf(mx, v[i]); }
+#pragma unroll
+        for (int o = 1; o < kPer; o <<= 1) {
+            mn = fminf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
+            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+        }
+        const float qmax = FMT == FMT_HQ8_G32 ? 255.0f : 15.0f;
+        const __half sh = __float2half_rn(__fdiv_rn(__fsub_rn(mx, mn), qmax));
+        const __half bh = __float2half_rn(mn);
+        const float es = __half2float(sh), eb = __half2float(bh);
+        const float safe = es > 0.0f ? es : 1.0f;
+        float far;
+        codes_fast(v, eb, safe, 0.0f, qmax, q, far);
+        if (far > 0.5f - (qmax + 2.0f) * kCodeErr) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) q[j] = static_cast<uint32_t>(fminf(fmaxf(rintf(__fdiv_rn(__fsub_rn(v[j], eb), safe)), 0.0f), qmax));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (FMT == FMT_HQ8_G32) word[j >> 2] |= (q[j] & 255u) << (8 * (j & 3));
+            else word[0] |= (q[j] & 15u) << (4 * j);   // byte i: elements 2 i (low nibble), 2 i + 1
+        }
+        if (!(es > 0.0f)) word[0] = word[1] = 0u;
+        hdr = static_cast<uint32_t>(__half_as_ushort(sh)) | (static_cast<uint32_t>(__half_as_ushort(bh)) << 16);
+    }
+    if (!live) return;
+    uint32_t* blk = reinterpret_cast<uint32_t*>(blocks + (c / kPer) * FmtTraits<FMT>::kBlockBytes);
+    const int sub = static_cast<int>(c % kPer);
+    if (sub == 0) blk[0] = hdr;
+    blk[1 + sub * ChunkGeom<FMT>::kWords] = word[0];
+    if (ChunkGeom<FMT>::kWords == 2) blk[2 + sub * 2] = word[1];
+}
+
+template <int FMT, bool VEC>
+__global__ void __launch_bounds__(256) qwc_quantize_kernel(const float* __restrict__ w, int64_t chunks, uint8_t* __restrict__ blocks,
+                                                           int32_t* status) {
+    constexpr int kU = 2;   // 64 bytes in flight per thread
+    const int lane = threadIdx.x & 31;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * 256;
+    for (int64_t c0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; c0 - lane < chunks; c0 += kU * step) {
+        float v[kU][8];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int64_t c = c0 + u * step;
+            if (c < chunks) {
+                if (VEC) {
+                    const float4 a = reinterpret_cast<const float4*>(w)[2 * c], b = reinterpret_cast<const float4*>(w)[2 * c + 1];
+                    v[u][0] = a.x; v[u][1] = a.y; v[u][2] = a.z; v[u][3] = a.w;
+                    v[u][4] = b.x; v[u][5] = b.y; v[u][6] = b.z; v[u][7] = b.w;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[u][i] = w[c * 8 + i];
+                }
             } else {
 #pragma unroll
-                for (int u = 0; u < T::kUnitsPerBlock; ++u) {
-                    uint32_t nib = q[u] << (4 * (lane & 1));
-                    nib |= __shfl_xor_sync(0xFFFFFFFFu, nib, 1);
-                    if ((lane & 1) == 0) blk[4 + 16 * u + (lane >> 1)] = static_cast<uint8_t>(nib);
-                }
+                for (int i = 0; i < 8; ++i) v[u][i] = 0.0f;
             }
-            if (lane == 0)
-                *reinterpret_cast<uint32_t*>(blk) = static_cast<uint32_t>(__half_as_ushort(sh)) |
-                                                    (static_cast<uint32_t>(__half_as_ushort(bh)) << 16);
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int64_t c = c0 + u * step;
+            if (c - lane < chunks) quantize_chunk<FMT>(v[u], lane, c, blocks, c < chunks);
+            // a weight that is not finite leaves no finite value in its rotated unit: only then look at the weights again
+            if (c < chunks && !(fabsf(v[u][0]) <= 3.402823466e38f)) {
+                bool finite = true;
+                for (int i = 0; i < 8; ++i) finite = finite && isfinite(w[c * 8 + i]);
+                if (!finite) atomicCAS(status, 0, QWC_DEV_NONFINITE_WEIGHT);
+            }
         }
     }
 }
 
+int chunk_grid(const qwc_hal* hal, int64_t chunks, int per_thread, int waves) {
+    int64_t g = (chunks + 256 * per_thread - 1) / (256 * per_thread);
+    const int64_t cap = static_cast<int64_t>(hal->sm_count) * waves;
+    if (g > cap) g = cap;
+    return static_cast<int>(g < 1 ? 1 : g);
+}
+
 template <int FMT>
 int launch_quantize(const qwc_hal* hal, cudaStream_t st, const float* w, int64_t n, int64_t k, void* blocks) {
-    const int64_t total = n * (k / FmtTraits<FMT>::kGroup);
-    if (total == 0) return QWC_OK;
-    int64_t grid = (total + 7) / 8;
-    const int64_t cap = static_cast<int64_t>(hal->sm_count) * 8;
-    if (grid > cap) grid = cap;
-    qwc_quantize_kernel<FMT><<<static_cast<unsigned>(grid), 256, 0, st>>>(w, n, k, static_cast<uint8_t*>(blocks), hal->status);
+    const int64_t chunks = n * (k / 8);
+    if (chunks == 0) return QWC_OK;
+    const int grid = chunk_grid(hal, chunks, 2, 16);
+    if (reinterpret_cast<uintptr_t>(w) % 16 == 0)
+        qwc_quantize_kernel<FMT, true><<<grid, 256, 0, st>>>(w, chunks, static_cast<uint8_t*>(blocks), hal->status);
+    else
+        qwc_quantize_kernel<FMT, false><<<grid, 256, 0, st>>>(w, chunks, static_cast<uint8_t*>(blocks), hal->status);
+    QWC_CUDA_TRY(cudaGetLastError());
+    return QWC_OK;
+}
+
+template <int FMT, typename OutT>
+int launch_dequant_out(const qwc_hal* hal, cudaStream_t st, const qwc_weight_view* w, void* out, int std_dom) {
+    const int64_t chunks = w->n * (w->k / 8);
+    if (chunks == 0) return QWC_OK;
+    const int grid = chunk_grid(hal, chunks, kUnroll, 16);
+    const uint8_t* p = static_cast<const uint8_t*>(w->blocks);
+    if (reinterpret_cast<uintptr_t>(out) % 16 == 0)
+        qwc_dequant_kernel<FMT, OutT, true><<<grid, 256, 0, st>>>(p, chunks, static_cast<OutT*>(out), std_dom);
+    else
+        qwc_dequant_kernel<FMT, OutT, false><<<grid, 256, 0, st>>>(p, chunks, static_cast<OutT*>(out), std_dom);
     QWC_CUDA_TRY(cudaGetLastError());
     return QWC_OK;
 }
 
 template <int FMT>
 int launch_dequant(const qwc_hal* hal, cudaStream_t st, const qwc_weight_view* w, void* out, int out_dtype, int std_dom) {
-    const int64_t total = w->n * (w->k / 32);
-    if (total == 0) return QWC_OK;
-    int64_t blocks = (total + 7) / 8;
-    const int64_t cap = static_cast<int64_t>(hal->sm_count) * 8;
-    if (blocks > cap) blocks = cap;
-    const uint8_t* p = static_cast<const uint8_t*>(w->blocks);
-    if (out_dtype == QWC_F32)
-        qwc_dequant_kernel<FMT, float><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p, w->n, w->k, static_cast<float*>(out), std_dom);
-    else
-        qwc_dequant_kernel<FMT, __half><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p, w->n, w->k, static_cast<__half*>(out), std_dom);
-    QWC_CUDA_TRY(cudaGetLastError());
-    return QWC_OK;
+    if (out_dtype == QWC_F32) return launch_dequant_out<FMT, float>(hal, st, w, out, std_dom);
+    return launch_dequant_out<FMT, __half>(hal, st, w, out, std_dom);
 }
 
 }  // namespace
@@ -203,11 +303,9 @@ int qwc_launch_dequant(const qwc_hal* hal, cudaStream_t st, const qwc_weight_vie
 
 int qwc_launch_fwht32_f16(const qwc_hal* hal, cudaStream_t st, void* x, int64_t count) {
     if (count == 0) return QWC_OK;
-    int64_t blocks = (count / 32 + 7) / 8;
-    const int64_t cap = static_cast<int64_t>(hal->sm_count) * 8;
-    if (blocks > cap) blocks = cap;
-    qwc_fwht32_f16_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<__half*>(x), count);
-    QWC_CUDA_TRY(cudaGetLastError());
+    const int64_t chunks = count / 8;
+    QWC_CUDA_TRY(qwc_launch_pdl(qwc_fwht32_f16_kernel, dim3(chunk_grid(hal, chunks, 1, 16)), dim3(256), 0, st, static_cast<__half*>(x), chunks,
+                                reinterpret_cast<uintptr_t>(x) % 16 == 0));
     return QWC_OK;
 }
 

@@ -441,52 +441,23 @@ qwc_gemv_stream_kernel(const GemvParams p, const __grid_constant__ CUtensorMap t
     };
     auto load_item = [&](const StageItem& si) {
         uint4 raw = make_uint4(0, 0, 0, 0);
-        if (si.live) {
-            if (vec_ok) raw = *reinterpret_cast<const uint4*>(si.src);
-            else {
-                __half tmp[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) tmp[i] = si.src[i];
-                raw = *reinterpret_cast<const uint4*>(tmp);
-            }
-        }
+        if (si.live) raw = load_f16x8(si.src, vec_ok);
         return raw;
     };
     auto finish_item = [&](const StageItem& si, uint4 raw) {
-        __half2 hv[4] = {*reinterpret_cast<__half2*>(&raw.x), *reinterpret_cast<__half2*>(&raw.y),
-                         *reinterpret_cast<__half2*>(&raw.z), *reinterpret_cast<__half2*>(&raw.w)};
-        if (!p.x_is_rotated) {
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { f[2 * i] = __low2float(hv[i]); f[2 * i + 1] = __high2float(hv[i]); }
-#pragma unroll
-            for (int h = 1; h < 8; h <<= 1)
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if ((i & h) == 0) {
-                        const float u = f[i], v = f[i + h];
-                        f[i] = __fadd_rn(u, v);
-                        f[i + h] = __fsub_rn(u, v);
-                    }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = fwht_xor_stage(f[i], 1, (t4 & 1) != 0);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = fwht_xor_stage(f[i], 2, (t4 & 2) != 0);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                hv[i] = __floats2half2_rn(__fmul_rn(f[2 * i], qwc_inv_sqrt32()), __fmul_rn(f[2 * i + 1], qwc_inv_sqrt32()));
-        }
+        if (!p.x_is_rotated) raw = fwht32_quad_f16(raw, t4);
+        const __half2* hv = reinterpret_cast<const __half2*>(&raw);
         if (si.live) {
             uint4 outv;
             if (FMT == FMT_HQ4_G64) {
                 // slot order inside a chunk: e0 e4 e1 e5 e2 e6 e3 e7
-                outv.x = __byte_perm(*reinterpret_cast<uint32_t*>(&hv[0]), *reinterpret_cast<uint32_t*>(&hv[2]), 0x5410);
-                outv.y = __byte_perm(*reinterpret_cast<uint32_t*>(&hv[0]), *reinterpret_cast<uint32_t*>(&hv[2]), 0x7632);
-                outv.z = __byte_perm(*reinterpret_cast<uint32_t*>(&hv[1]), *reinterpret_cast<uint32_t*>(&hv[3]), 0x5410);
-                outv.w = __byte_perm(*reinterpret_cast<uint32_t*>(&hv[1]), *reinterpret_cast<uint32_t*>(&hv[3]), 0x7632);
+                outv.x = __byte_perm(*reinterpret_cast<const uint32_t*>(&hv[0]), *reinterpret_cast<const uint32_t*>(&hv[2]), 0x5410);
+                outv.y = __byte_perm(*reinterpret_cast<const uint32_t*>(&hv[0]), *reinterpret_cast<const uint32_t*>(&hv[2]), 0x7632);
+                outv.z = __byte_perm(*reinterpret_cast<const uint32_t*>(&hv[1]), *reinterpret_cast<const uint32_t*>(&hv[3]), 0x5410);
+                outv.w = __byte_perm(*reinterpret_cast<const uint32_t*>(&hv[1]), *reinterpret_cast<const uint32_t*>(&hv[3]), 0x7632);
             } else {
-                outv = make_uint4(*reinterpret_cast<uint32_t*>(&hv[0]), *reinterpret_cast<uint32_t*>(&hv[1]),
-                                  *reinterpret_cast<uint32_t*>(&hv[2]), *reinterpret_cast<uint32_t*>(&hv[3]));
+                outv = make_uint4(*reinterpret_cast<const uint32_t*>(&hv[0]), *reinterpret_cast<const uint32_t*>(&hv[1]),
+                                  *reinterpret_cast<const uint32_t*>(&hv[2]), *reinterpret_cast<const uint32_t*>(&hv[3]));
             }
             *reinterpret_cast<uint4*>(xs + x_offset<FMT>(si.tok, si.unit, t4, p.units)) = outv;
         }

@@ -132,6 +132,30 @@ def test_device_quantizer_bytes_equal_the_packer(hal, oracle, golden, name):
     assert np.array_equal(got, oracle.quantize(w, oracle.FORMATS[name]).reshape(-1))
 
 
+# Chunks of eight elements: planes of one unit, of less than a warp, and of one chunk more than a grid step's worth per thread;
+# weights and outputs that are not 16-byte aligned; weights on a grid where many quotients fall on or next to a rounding point.
+@pytest.mark.parametrize("name", FMTS)
+@pytest.mark.parametrize("n,k", [(1, 64), (3, 64), (5, 4096), (149, 1024)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_codec_chunk_edges(hal, oracle, name, n, k, shift):
+    import qwegn_b200 as q
+    fmt = oracle.FORMATS[name]
+    rng = np.random.default_rng(n + k + shift)
+    w = rng.normal(0.0, 0.02, (n, k)).astype(np.float32)
+    w[0] = oracle.fwht32(rng.integers(-15, 16, (1, k)).astype(np.float32) * np.float32(0.0078125))[0]
+    buf = torch.zeros(n * k + shift, dtype=torch.float32, device="cuda")
+    buf[shift:] = torch.from_numpy(w).cuda().reshape(-1)
+    bank = q.QWGemm.quantize(hal, buf[shift:].view(n, k), q.CONTAINERS[name])
+    blocks = oracle.quantize(w, fmt)
+    assert np.array_equal(bank.cpu().numpy(), blocks.reshape(-1))
+    view = q.QWWeightView(bank, n, k, q.CONTAINERS[name])
+    ref = oracle.dequant(blocks, fmt)
+    for dt in (torch.float16, torch.float32):
+        out = torch.zeros(n * k + shift, dtype=dt, device="cuda")
+        q.QWGemm.dequant(hal, view, out[shift:])
+        assert np.array_equal(out[shift:].cpu().numpy(), ref.reshape(-1).astype(out.cpu().numpy().dtype))
+
+
 def test_aq_quantizer_golden_on_device(hal, golden):
     import qwegn_b200 as q
     g = golden["ref_fixtures"]
