@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(1024) qwc_rmsnorm_fwht_kernel(const __half* __
                                                                 int rotate) {
     __shared__ float s_part[32];
     __shared__ float s_rstd;
+    pdl_enter();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x;
     const int chunks = hidden / 8;
     const int64_t row = blockIdx.x;
@@ -83,23 +84,7 @@ __global__ void __launch_bounds__(1024) qwc_rmsnorm_fwht_kernel(const __half* __
                 f[2 * j] = __fmul_rn(__fmul_rn(fv.x, rstd), __fadd_rn(gv.x, 1.0f));
                 f[2 * j + 1] = __fmul_rn(__fmul_rn(fv.y, rstd), __fadd_rn(gv.y, 1.0f));
             }
-            if (rotate) {
-#pragma unroll
-                for (int hh = 1; hh < 8; hh <<= 1)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if ((j & hh) == 0) {
-                            const float a = f[j], b = f[j + hh];
-                            f[j] = __fadd_rn(a, b);
-                            f[j + hh] = __fsub_rn(a, b);
-                        }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = fwht_xor_stage(f[j], 1, (t4 & 1) != 0);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = fwht_xor_stage(f[j], 2, (t4 & 2) != 0);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = __fmul_rn(f[j], qwc_inv_sqrt32());
-            }
+            if (rotate) fwht32_quad(f, t4);
             uint4 o;
             __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
@@ -112,6 +97,7 @@ __global__ void __launch_bounds__(1024) qwc_rmsnorm_fwht_kernel(const __half* __
 // The explicit f32 -> f16 cast seam between the f32-emitting GEMV doors and the f16 engine storage
 // (QWGemm.encodeCast, Sources/Operators/QWGEMM/QWGemm.swift:302-320): 8 elements per thread, round to nearest even.
 __global__ void __launch_bounds__(256) qwc_cast_f32_to_f16_kernel(const float4* __restrict__ x, uint4* __restrict__ y, int64_t n8) {
+    pdl_enter();
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const float4 a = x[2 * i], b = x[2 * i + 1];
         uint4 o;
@@ -142,6 +128,7 @@ __global__ void __launch_bounds__(1024) qwc_head_argmax_kernel(const float* __re
                                                                int32_t* __restrict__ tokens) {
     __shared__ unsigned long long s_best[32];
     __shared__ unsigned long long s_cluster[kArgmaxCluster];
+    pdl_enter();
     cg::cluster_group cluster = cg::this_cluster();
     const int crank = static_cast<int>(cluster.block_rank());
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -210,9 +197,8 @@ extern "C" int qwc_cast_f32_to_f16(qwc_hal* hal, qwc_stream stream, const float*
     int64_t blocks = (n8 + 255) / 256;
     const int64_t cap = static_cast<int64_t>(hal->sm_count) * 8;
     if (blocks > cap) blocks = cap;
-    qwc_cast_f32_to_f16_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const float4*>(x_f32), static_cast<uint4*>(y_f16), n8);
-    QWC_CUDA_TRY(cudaGetLastError());
+    QWC_CUDA_TRY(qwc_launch_pdl(qwc_cast_f32_to_f16_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                reinterpret_cast<const float4*>(x_f32), static_cast<uint4*>(y_f16), n8));
     return QWC_OK;
 }
 
@@ -224,7 +210,9 @@ extern "C" int qwc_head_argmax(qwc_hal* hal, qwc_stream stream, const float* log
     if (rows < 0) return qwc_fail(QWC_ERR_BAD_SHAPE, "rows is negative");
     if (rows == 0) return QWC_OK;
     if (!logits || !tokens) return qwc_fail(QWC_ERR_BAD_SHAPE, "null buffer");
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kArgmaxCluster;
     attr[0].val.clusterDim.y = 1;
@@ -236,7 +224,7 @@ extern "C" int qwc_head_argmax(qwc_hal* hal, qwc_stream stream, const float* log
         cfg.blockDim = dim3(1024, 1, 1);
         cfg.stream = static_cast<cudaStream_t>(stream);
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         QWC_CUDA_TRY(cudaLaunchKernelEx(&cfg, qwc_head_argmax_kernel, logits + r0 * ld, ld, static_cast<int>(n), tokens + r0));
     }
     return QWC_OK;
@@ -262,9 +250,8 @@ extern "C" int qwc_rmsnorm_fwht(qwc_hal* hal, qwc_stream stream, const void* x_f
     if (threads < 32) threads = 32;
     // more threads than strictly needed (up to one chunk per thread) shorten a row's latency at decode
     while (threads * 2 <= chunks && threads * 2 <= 1024) threads *= 2;
-    qwc_rmsnorm_fwht_kernel<<<static_cast<unsigned>(rows), threads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(x_f16), static_cast<const __half*>(gamma_f16), static_cast<__half*>(y_f16),
-        static_cast<__half*>(residual_f16), static_cast<int>(hidden), eps, rotate);
-    QWC_CUDA_TRY(cudaGetLastError());
+    QWC_CUDA_TRY(qwc_launch_pdl(qwc_rmsnorm_fwht_kernel, dim3(static_cast<unsigned>(rows)), dim3(threads), 0, static_cast<cudaStream_t>(stream),
+                                static_cast<const __half*>(x_f16), static_cast<const __half*>(gamma_f16), static_cast<__half*>(y_f16),
+                                static_cast<__half*>(residual_f16), static_cast<int>(hidden), eps, rotate));
     return QWC_OK;
 }
