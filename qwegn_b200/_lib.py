@@ -54,6 +54,21 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
+
+
+def host():
+    """The _qwchost extension (native side of the doors); raises if it was not built."""
+    global _host
+    if _host is None:
+        load()   # the extension's own library reference then resolves to the one that is loaded
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        try:
+            from . import _qwchost
+        except ImportError as e:
+            raise RuntimeError(f"the _qwchost extension is missing or does not load ({e}): build it with `python -m qwegn_b200.build`") from e
+        _host = _qwchost
+    return _host
 
 
 def load() -> ctypes.CDLL:

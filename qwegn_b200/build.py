@@ -1,4 +1,4 @@
-"""Builds libqwcuda.so in place with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds libqwcuda.so (nvcc, sm_100a; cross-compiles without a GPU) and the _qwchost extension over it in place.
 
     python -m qwegn_b200.build [--force] [--verbose]
 """
@@ -8,6 +8,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
@@ -44,7 +45,34 @@ def is_stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+HOST_SRC = os.path.join(CSRC, "qwc_host.cpp")
+HOST_PATH = os.path.join(PKG_DIR, "_qwchost" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_host(force: bool = False) -> str:
+    """The native side of the Python doors: tensor checks and the library call in one C function (qwc_host.cpp)."""
+    deps = [HOST_SRC, os.path.join(CSRC, HEADERS[1])]
+    if not force and os.path.exists(HOST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_PATH) for d in deps):
+        return HOST_PATH
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cmd = [os.environ.get("CXX", "g++"), "-shared", "-fPIC", "-O2", "-std=c++17", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I" + sysconfig.get_paths()["include"], "-isystem", os.path.join(base, "include"), "-isystem",
+           os.path.join(base, "include", "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda, "include"), HOST_SRC,
+           "-o", HOST_PATH, "-L" + PKG_DIR, "-l:libqwcuda.so", "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(base, "lib"),
+           "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
+    subprocess.check_call(cmd)
+    return HOST_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_library(force, verbose)
+    build_host(force)
+    return LIB_PATH
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not is_stale():
         return LIB_PATH
     objs = []
@@ -67,7 +95,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + out)
         if verbose or "warning" in out:
             sys.stderr.write(out)
-    link = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-Xcompiler", "-fPIC", "-lcudart"]
+    link = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-Xcompiler", "-fPIC", "-lcudart", "-Xlinker", "-soname=libqwcuda.so"]
     subprocess.check_call(link)
     return LIB_PATH
 

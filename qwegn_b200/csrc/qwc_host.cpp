@@ -1,0 +1,289 @@
+// Native side of the Python doors: the tensor checks, the stream lookup and the call into the C ABI of one encode call in one
+// C function.  A decode step makes a few calls of 5-10 us of device time each per layer; the same checks through tensor
+// attributes and ctypes cost 9-10 us of host time per call, i.e. they, not the kernels, set the pace of every loop that is not
+// captured in a graph.
+//
+// Every function returns the C ABI's status, or kRecheck when a tensor does not qualify (type, device, layout, extents):
+// the Python door then runs its own checks, which raise the error.  The library call runs without the GIL, as under ctypes.
+#include <Python.h>
+
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+
+#include "../../include/qwc.h"
+
+namespace {
+
+constexpr long kRecheck = -1;
+
+struct Args {
+    PyObject* const* a;
+    Py_ssize_t n;
+    bool ok = true;
+    int64_t i64(int k) {
+        const long long v = PyLong_AsLongLong(a[k]);
+        if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); ok = false; }
+        return v;
+    }
+    void* ptr(int k) { return reinterpret_cast<void*>(static_cast<uintptr_t>(i64(k))); }
+    double f64(int k) {
+        const double v = PyFloat_AsDouble(a[k]);
+        if (v == -1.0 && PyErr_Occurred()) { PyErr_Clear(); ok = false; }
+        return v;
+    }
+    bool truth(int k) {
+        const int v = PyObject_IsTrue(a[k]);
+        if (v < 0) { PyErr_Clear(); ok = false; }
+        return v > 0;
+    }
+    const at::Tensor* tensor(int k) {
+        if (!THPVariable_Check(a[k])) { ok = false; return nullptr; }
+        return &THPVariable_Unpack(a[k]);
+    }
+    bool none(int k) const { return a[k] == Py_None; }
+    // a torch.cuda.Stream, or None for the current stream of the current device
+    qwc_stream stream(int k) {
+        if (none(k)) return static_cast<cudaStream_t>(c10::cuda::getCurrentCUDAStream());
+        PyObject* v = PyObject_GetAttrString(a[k], "cuda_stream");
+        const long long p = v ? PyLong_AsLongLong(v) : 0;
+        Py_XDECREF(v);
+        if (PyErr_Occurred()) { PyErr_Clear(); ok = false; }
+        return reinterpret_cast<qwc_stream>(static_cast<uintptr_t>(p));
+    }
+};
+
+PyObject* done(long rc) { return PyLong_FromLong(rc); }
+PyObject* recheck() { return PyLong_FromLong(kRecheck); }
+
+template <typename F> PyObject* call(F&& f) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = f();
+    Py_END_ALLOW_THREADS
+    return done(rc);
+}
+
+bool on(const at::Tensor& t, int64_t dev) { return t.is_cuda() && t.get_device() == dev; }
+bool f16(const at::Tensor& t) { return t.scalar_type() == at::kHalf; }
+bool f32(const at::Tensor& t) { return t.scalar_type() == at::kFloat; }
+int32_t dt(const at::Tensor& t) { return f16(t) ? QWC_F16 : QWC_F32; }
+
+// A vector or matrix seen as rows: extents and row stride (a vector is one row; `flat`: so is a contiguous tensor of more
+// dimensions).
+struct Rows {
+    int64_t m, n, ld;
+    bool ok;
+    explicit Rows(const at::Tensor& t, bool flat = false) : m(0), n(0), ld(0), ok(false) {
+        if (t.dim() == 1) {
+            m = 1; n = t.size(0); ld = n;
+            ok = n <= 1 || t.stride(0) == 1;
+        } else if (t.dim() == 2) {
+            m = t.size(0); n = t.size(1); ld = t.stride(0);
+            ok = t.stride(1) == 1;
+        } else if (flat && t.is_contiguous()) {
+            m = 1; n = ld = t.numel();
+            ok = true;
+        }
+    }
+};
+
+// encode(hal, device, view, bank, x, y, epi, x_is_rotated, stream, workspace)
+PyObject* gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 10) return recheck();
+    Args g{a, n};
+    const int64_t dev = g.i64(1);
+    auto* w = static_cast<const qwc_weight_view*>(g.ptr(2));
+    const at::Tensor *bank = g.tensor(3), *x = g.tensor(4), *y = g.tensor(5);
+    if (!g.ok || !on(*bank, dev) || !on(*x, dev) || !on(*y, dev) || !f16(*x) || !(f16(*y) || f32(*y))) return recheck();
+    const int32_t epi = static_cast<int32_t>(g.i64(6)), rot = g.truth(7);
+    const Rows rx(*x), ry(*y);
+    const int64_t n_out = epi == QWC_EPI_NONE ? w->n : w->n / 2;
+    if (!rx.ok || !ry.ok || rx.n != w->k || ry.m != rx.m || ry.n != n_out) return recheck();
+    const int64_t m = rx.m;
+    if (m > 1 && (rx.ld < w->k || ry.ld < n_out)) return recheck();
+    const int64_t ldx = m > 1 ? rx.ld : std::max(rx.ld, w->k), ldy = m > 1 ? ry.ld : std::max(ry.ld, n_out);
+    const qwc_stream st = g.stream(8);
+    void* ws = nullptr;
+    size_t ws_bytes = 0;
+    if (!g.none(9)) {
+        const at::Tensor* t = g.tensor(9);
+        if (t == nullptr || !on(*t, dev) || !t->is_contiguous()) return recheck();
+        ws = t->data_ptr();
+        ws_bytes = t->nbytes();
+    }
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    const void* xp = x->data_ptr();
+    void* yp = y->data_ptr();
+    const int32_t yd = dt(*y);
+    return call([&] { return qwc_gemm(hal, st, w, xp, m, ldx, yp, yd, ldy, epi, rot, ws, ws_bytes); });
+}
+
+// encodeHQ4F32V4(hal, view, x, y, rows, epi, scale, x_is_rotated, workspace, stream)
+PyObject* gemm_f32(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 10) return recheck();
+    Args g{a, n};
+    auto* w = static_cast<const qwc_weight_view*>(g.ptr(1));
+    const at::Tensor *x = g.tensor(2), *y = g.tensor(3), *ws = g.tensor(8);
+    if (!g.ok || !f32(*x) || !x->is_cuda() || !(f16(*y) || f32(*y)) || !y->is_cuda()) return recheck();
+    const int64_t rows = g.i64(4);
+    const Rows rx(*x, true), ry(*y, true);
+    if (!rx.ok || !ry.ok || rx.m != rows || ry.m != rows || rx.n != w->k || ry.n != w->n) return recheck();
+    const int32_t epi = static_cast<int32_t>(g.i64(5)), rot = g.truth(7);
+    const float scale = static_cast<float>(g.f64(6));
+    const qwc_stream st = g.stream(9);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    const float* xp = static_cast<const float*>(x->data_ptr());
+    void *yp = y->data_ptr(), *wp = ws->data_ptr();
+    const size_t wb = ws->nbytes();
+    const int64_t ldx = rows > 1 ? rx.ld : w->k, ldy = rows > 1 ? ry.ld : w->n;
+    const int32_t yd = dt(*y);
+    return call([&] { return qwc_gemm_f32(hal, st, w, xp, rows, ldx, yp, yd, ldy, epi, scale, rot, wp, wb); });
+}
+
+// encodeRMSNorm(hal, x, gamma, out, eps, residual, rotate, stream)
+PyObject* rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 8) return recheck();
+    Args g{a, n};
+    const at::Tensor *x = g.tensor(1), *gamma = g.tensor(2), *out = g.tensor(3), *res = g.none(5) ? nullptr : g.tensor(5);
+    if (!g.ok) return recheck();
+    for (const at::Tensor* t : {x, gamma, out, res})
+        if (t != nullptr && (!f16(*t) || !t->is_cuda() || !t->is_contiguous())) return recheck();
+    const int64_t rows = x->dim() == 2 ? x->size(0) : 1, hidden = x->dim() == 2 ? x->size(1) : x->numel();
+    if (gamma->numel() != hidden || out->numel() != x->numel() || (res != nullptr && res->numel() != x->numel())) return recheck();
+    const float eps = static_cast<float>(g.f64(4));
+    const int32_t rotate = g.truth(6);
+    const qwc_stream st = g.stream(7);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    const void *xp = x->data_ptr(), *gp = gamma->data_ptr();
+    void *op = out->data_ptr(), *rp = res != nullptr ? res->data_ptr() : nullptr;
+    return call([&] { return qwc_rmsnorm_fwht(hal, st, xp, gp, op, rp, rows, hidden, eps, rotate); });
+}
+
+// encodeArgmax(hal, logits, tokens, stream)
+PyObject* argmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 4) return recheck();
+    Args g{a, n};
+    const at::Tensor *l = g.tensor(1), *tok = g.tensor(2);
+    if (!g.ok || !f32(*l) || tok->scalar_type() != at::kInt || !l->is_cuda()) return recheck();
+    const Rows r(*l, true);
+    if (!r.ok) return recheck();
+    const qwc_stream st = g.stream(3);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    const float* lp = static_cast<const float*>(l->data_ptr());
+    auto* tp = static_cast<int32_t*>(tok->data_ptr());
+    const int64_t ld = r.m > 1 ? r.ld : r.n;
+    return call([&] { return qwc_head_argmax(hal, st, lp, ld, r.m, r.n, tp); });
+}
+
+// encodeFnRouterGemm(hal, weight, x, y, stream)
+PyObject* router(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 5) return recheck();
+    Args g{a, n};
+    const at::Tensor *w = g.tensor(1), *x = g.tensor(2), *y = g.tensor(3);
+    if (!g.ok || !(f16(*w) || f32(*w) || w->scalar_type() == at::kBFloat16) || !(f16(*x) || f32(*x)) || !f32(*y)) return recheck();
+    if (!w->is_contiguous() || !y->is_contiguous() || w->dim() != 2 || x->dim() != 2 || y->dim() != 2 || x->stride(1) != 1) return recheck();
+    const int64_t t = x->size(0), h = x->size(1), e = w->size(0);
+    if (w->size(1) != h || y->size(0) != t || y->size(1) != e) return recheck();
+    const qwc_stream st = g.stream(4);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    const void *xp = x->data_ptr(), *wp = w->data_ptr();
+    auto* yp = static_cast<float*>(y->data_ptr());
+    const int32_t xd = dt(*x), wd = w->scalar_type() == at::kBFloat16 ? QWC_BF16 : dt(*w);
+    const int64_t ldx = x->stride(0);
+    return call([&] { return qwc_moe_router_gemm(hal, st, xp, xd, ldx, t, h, wp, wd, e, yp); });
+}
+
+// encodeResident(hal, device, bank_gu, bank_dn, experts, inter, top_k, norm_topk, routed_scale, x, logits, out, scratch, x_is_rotated, stream)
+PyObject* moe(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 15) return recheck();
+    Args g{a, n};
+    const int64_t dev = g.i64(1), e = g.i64(4), inter = g.i64(5), k = g.i64(6);
+    auto *gu = static_cast<const qwc_weight_view*>(g.ptr(2)), *dn = static_cast<const qwc_weight_view*>(g.ptr(3));
+    const at::Tensor *x = g.tensor(9), *l = g.tensor(10), *out = g.tensor(11), *sc = g.tensor(12);
+    if (!g.ok || !on(*x, dev) || !on(*l, dev) || !on(*out, dev) || !on(*sc, dev)) return recheck();
+    if (!f16(*x) || !f32(*l) || !(f16(*out) || f32(*out)) || sc->scalar_type() != at::kByte) return recheck();
+    if (x->dim() != 2 || x->stride(1) != 1 || x->size(1) != gu->k || (x->size(0) > 1 && x->stride(0) < gu->k)) return recheck();
+    const int64_t t = x->size(0), h = gu->k, ldx = x->stride(0);
+    if (!l->is_contiguous() || l->dim() != 2 || l->size(0) != t || l->size(1) != e) return recheck();
+    if (!out->is_contiguous() || out->dim() != 2 || out->size(0) != t || out->size(1) != h || !sc->is_contiguous()) return recheck();
+    if (static_cast<size_t>(sc->numel()) < qwc_moe_scratch_bytes(t, e, k, h, inter)) return recheck();
+    const int32_t norm = g.truth(7), rot = g.truth(13);
+    const float scale = static_cast<float>(g.f64(8));
+    const qwc_stream st = g.stream(14);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    const void* xp = x->data_ptr();
+    const float* lp = static_cast<const float*>(l->data_ptr());
+    void *op = out->data_ptr(), *sp = sc->data_ptr();
+    const int32_t od = dt(*out);
+    const size_t sb = sc->nbytes();
+    return call([&] { return qwc_moe_forward(hal, st, gu, dn, e, inter, xp, t, ldx, rot, lp, k, norm, scale, op, od, sp, sb); });
+}
+
+// quantize(hal, w, kind, bits, group, out, block_bytes, stream)
+PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 8) return recheck();
+    Args g{a, n};
+    const at::Tensor *w = g.tensor(1), *out = g.tensor(5);
+    if (!g.ok || !f32(*w) || !w->is_cuda() || !w->is_contiguous() || w->dim() != 2) return recheck();
+    const int32_t kind = static_cast<int32_t>(g.i64(2)), bits = static_cast<int32_t>(g.i64(3)), group = static_cast<int32_t>(g.i64(4));
+    const int64_t rows = w->size(0), k = w->size(1), need = g.i64(6);
+    if (group <= 0 || k % group != 0 || out->scalar_type() != at::kByte || !out->is_contiguous()) return recheck();
+    if (out->numel() < rows * (k / group) * need) return recheck();   // need: bytes of a block
+    const qwc_stream st = g.stream(7);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    const float* wp = static_cast<const float*>(w->data_ptr());
+    void* op = out->data_ptr();
+    return call([&] { return qwc_quantize(hal, st, wp, rows, k, kind, bits, group, op); });
+}
+
+// dequant(hal, view, out, standard_domain, stream)
+PyObject* dequant(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 5) return recheck();
+    Args g{a, n};
+    auto* w = static_cast<const qwc_weight_view*>(g.ptr(1));
+    const at::Tensor* out = g.tensor(2);
+    if (!g.ok || !(f16(*out) || f32(*out)) || !out->is_cuda() || !out->is_contiguous() || out->numel() != w->n * w->k) return recheck();
+    const int32_t std_dom = g.truth(3);
+    const qwc_stream st = g.stream(4);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    void* op = out->data_ptr();
+    const int32_t od = dt(*out);
+    return call([&] { return qwc_dequant(hal, st, w, op, od, std_dom); });
+}
+
+// encodeFwht32(hal, x, stream)
+PyObject* fwht32(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 3) return recheck();
+    Args g{a, n};
+    const at::Tensor* x = g.tensor(1);
+    if (!g.ok || !f16(*x) || !x->is_cuda() || !x->is_contiguous()) return recheck();
+    const qwc_stream st = g.stream(2);
+    if (!g.ok) return recheck();
+    auto* hal = static_cast<qwc_hal*>(g.ptr(0));
+    void* xp = x->data_ptr();
+    const int64_t count = x->numel();
+    return call([&] { return qwc_fwht32_f16(hal, st, xp, count); });
+}
+
+#define QWC_DOOR(name, doc) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, doc}
+PyMethodDef kMethods[] = {
+    QWC_DOOR(gemm, "QWGemm.encode"), QWC_DOOR(gemm_f32, "QWGemm.encodeHQ4F32V4"), QWC_DOOR(rmsnorm, "QWGemm.encodeRMSNorm"),
+    QWC_DOOR(argmax, "QWGemm.encodeArgmax"), QWC_DOOR(router, "QWGemmMoE.encodeFnRouterGemm"), QWC_DOOR(moe, "QWMoEOperator.encodeResident"),
+    QWC_DOOR(quantize, "QWGemm.quantize"), QWC_DOOR(dequant, "QWGemm.dequant"), QWC_DOOR(fwht32, "QWGemm.encodeFwht32"),
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_qwchost", "Native side of the Python doors.", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__qwchost() { return PyModule_Create(&kModule); }

@@ -74,6 +74,8 @@ class QWHal:
         _check(lib.qwc_hal_create(device, ctypes.byref(h)))
         self._h = h
         self._lib = lib
+        self._addr, self._index = h.value, device   # what the native doors take
+        _native()
 
     @property
     def handle(self) -> ctypes.c_void_p:
@@ -104,6 +106,27 @@ class QWHal:
             self.close()
         except Exception:
             pass
+
+
+_nat = None
+
+
+def _native():
+    """The native doors (csrc/qwc_host.cpp), loaded with the first QWHal.  They answer -1 where a tensor does not qualify; the
+    Python door then runs its own checks, which raise."""
+    global _nat
+    if _nat is None:
+        _nat = _lib.host()
+    return _nat
+
+
+def _refused(rc: int, door: str) -> None:
+    """Ends a native call: rc 0 returns, a library status raises, -1 left by checks that found nothing raises too."""
+    if rc == 0:
+        return
+    if rc > 0:
+        _check(rc)
+    raise QWGemmError(3, f"{door}: a tensor does not qualify")
 
 
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> ctypes.c_void_p:
@@ -163,6 +186,7 @@ class QWWeightView:
         self.bank = blocks
         self.container = container
         self.c = WeightViewC()
+        self._addr = ctypes.addressof(self.c)
         avail = blocks.numel() - byte_offset
         if avail < 0:
             raise QWGemmError(2, "byte offset beyond the bank")
@@ -213,13 +237,16 @@ class QWGemm:
                x_is_rotated: bool = False, stream: Optional[torch.cuda.Stream] = None,
                workspace: Optional[torch.Tensor] = None) -> None:
         """y[m, n_out] = epilogue(rot(x) . W_rot^T).  x f16 [m, k] (or [k]); y f16/f32 [m, n_out] (or [n_out])."""
-        x2, y2, m, n_out, ldx, ldy = check_matmul_tensors(hal, w, x, y, epi)
-        ws_ptr, ws_bytes = None, 0
-        if workspace is not None:
-            check_device_tensor(hal, workspace, "workspace", workspace.dtype)
-            ws_ptr, ws_bytes = workspace.data_ptr(), workspace.numel() * workspace.element_size()
-        _check(_lib.load().qwc_gemm(hal.handle, _stream_ptr(stream), ctypes.byref(w.c), x2.data_ptr(), m, ldx, y2.data_ptr(),
-                                    F16 if y.dtype == torch.float16 else F32, ldy, epi, int(x_is_rotated), ws_ptr, ws_bytes))
+        try:
+            rc = _nat.gemm(hal._addr, hal._index, w._addr, w.bank, x, y, epi, x_is_rotated, stream, workspace)
+        except AttributeError:   # a stand-in for the device context or the view: the checks below refuse it by its tensors
+            rc = -1
+        if rc:
+            if rc < 0:
+                check_matmul_tensors(hal, w, x, y, epi)
+                if workspace is not None:
+                    check_device_tensor(hal, workspace, "workspace", workspace.dtype)
+            _refused(rc, "encode")
 
     # The reference's f16-store door (QWGemm.swift:137) is the same call with an f16 output tensor.
     encodeH16 = encode
@@ -239,6 +266,11 @@ class QWGemm:
         """f32-activation matmul (QWGemmF32.swift:143-199; encodeHQ4F32BM :309-350 is the same call with more rows).
         x f32 [rows, k] in the rotated basis (the reference's dataflow; x_is_rotated=False rotates here in f32);
         epi 0 none, 1 silu(y/scale), 2 sigmoid, 3 silu(y/scale) + FWHT-32; y f16/f32 [rows, n]."""
+        rc = _nat.gemm_f32(hal._addr, w._addr, x, y, rows, epi, scale, x_is_rotated, workspace, stream)
+        if rc == 0:
+            return
+        if rc > 0:
+            _check(rc)
         if x.dtype != torch.float32 or not x.is_cuda or y.dtype not in (torch.float16, torch.float32) or not y.is_cuda:
             raise QWGemmError(3, "x must be CUDA float32, y CUDA float16/float32")
         x2 = x if x.dim() == 2 else x.view(1, -1)
@@ -249,20 +281,17 @@ class QWGemm:
             raise QWGemmError(3, f"x is {tuple(x2.shape)}, y {tuple(y2.shape)}; the bank is n={w.n}, k={w.k}")
         if workspace is None:
             raise QWGemmError(3, "the f32 door needs a workspace of f32WorkspaceBytes() bytes")
-        _check(_lib.load().qwc_gemm_f32(hal.handle, _stream_ptr(stream), ctypes.byref(w.c), x2.data_ptr(), rows,
-                                        x2.stride(0) if rows > 1 else w.k, y2.data_ptr(),
-                                        F16 if y.dtype == torch.float16 else F32, y2.stride(0) if rows > 1 else w.n,
-                                        epi, float(scale), int(x_is_rotated), workspace.data_ptr(),
-                                        workspace.numel() * workspace.element_size()))
+        _refused(rc, "encodeHQ4F32V4")
 
     encodeHQ4F32BM = encodeHQ4F32V4
 
     @staticmethod
     def encodeFwht32(hal: QWHal, x: torch.Tensor, stream: Optional[torch.cuda.Stream] = None) -> None:
         """In-place activation rotation (QWGemm.swift:285-300)."""
-        if x.dtype != torch.float16 or not x.is_cuda or not x.is_contiguous():
+        rc = _nat.fwht32(hal._addr, x, stream)
+        if rc < 0 and (x.dtype != torch.float16 or not x.is_cuda or not x.is_contiguous()):
             raise QWGemmError(3, "x must be a contiguous CUDA float16 tensor")
-        _check(_lib.load().qwc_fwht32_f16(hal.handle, _stream_ptr(stream), x.data_ptr(), x.numel()))
+        _refused(rc, "encodeFwht32")
 
     @staticmethod
     def encodeCast(hal: QWHal, x32: torch.Tensor, y16: torch.Tensor, stream: Optional[torch.cuda.Stream] = None) -> None:
@@ -276,11 +305,10 @@ class QWGemm:
     @staticmethod
     def encodeArgmax(hal: QWHal, logits: torch.Tensor, tokens: torch.Tensor, stream: Optional[torch.cuda.Stream] = None) -> None:
         """Greedy token per row of f32 logits [rows, vocab] in the reference's key order (QWGemmF32.swift:201-307)."""
-        if logits.dtype != torch.float32 or tokens.dtype != torch.int32 or not logits.is_cuda or logits.stride(-1) != 1:
+        rc = _nat.argmax(hal._addr, logits, tokens, stream)
+        if rc < 0 and (logits.dtype != torch.float32 or tokens.dtype != torch.int32 or not logits.is_cuda or logits.stride(-1) != 1):
             raise QWGemmError(3, "logits must be CUDA float32 with contiguous rows, tokens int32")
-        l2 = logits if logits.dim() == 2 else logits.view(1, -1)
-        _check(_lib.load().qwc_head_argmax(hal.handle, _stream_ptr(stream), l2.data_ptr(), l2.stride(0) if l2.shape[0] > 1 else l2.shape[1],
-                                           l2.shape[0], l2.shape[1], tokens.data_ptr()))
+        _refused(rc, "encodeArgmax")
 
     @staticmethod
     def encodeRMSNorm(hal: QWHal, x: torch.Tensor, gamma: torch.Tensor, out: torch.Tensor, eps: float = 1e-6,
@@ -289,33 +317,39 @@ class QWGemm:
         """RMSNorm with (1 + gamma) and rotated f16 output, optionally fused with residual += x (the driver's
         encodeRMSNormFast / encodeRMSNormResidualFast, Sources/Runtime/QWEngine/Driver/EncodeKernels.swift:339-404).
         Feed `out` to encode(..., x_is_rotated=True)."""
+        rc = _nat.rmsnorm(hal._addr, x, gamma, out, eps, residual, rotate, stream)
+        if rc == 0:
+            return
+        if rc > 0:
+            _check(rc)
         for t in (x, gamma, out) + ((residual,) if residual is not None else ()):
             if t.dtype != torch.float16 or not t.is_cuda or not t.is_contiguous():
                 raise QWGemmError(3, "norm tensors must be contiguous CUDA float16")
-        x2 = x if x.dim() == 2 else x.view(1, -1)
-        rows, hidden = x2.shape
-        if gamma.numel() != hidden or out.numel() != x.numel() or (residual is not None and residual.numel() != x.numel()):
-            raise QWGemmError(3, "shape mismatch")
-        _check(_lib.load().qwc_rmsnorm_fwht(hal.handle, _stream_ptr(stream), x.data_ptr(), gamma.data_ptr(), out.data_ptr(),
-                                            None if residual is None else residual.data_ptr(), rows, hidden, float(eps),
-                                            int(rotate)))
+        raise QWGemmError(3, "shape mismatch")
 
     @staticmethod
     def dequant(hal: QWHal, w: QWWeightView, out: torch.Tensor, standard_domain: bool = False,
                 stream: Optional[torch.cuda.Stream] = None) -> None:
         """Device twin of Pack.dequantHQ4Slab / dequantHQBlockSlab (Sources/Foundation/QWQuant/QWPack.swift:205-321)."""
-        if out.dtype not in (torch.float16, torch.float32) or not out.is_cuda or not out.is_contiguous():
-            raise QWGemmError(3, "out must be a contiguous CUDA float16/float32 tensor")
-        if out.numel() != w.n * w.k:
-            raise QWGemmError(3, f"out has {out.numel()} elements, expected {w.n * w.k}")
-        _check(_lib.load().qwc_dequant(hal.handle, _stream_ptr(stream), ctypes.byref(w.c), out.data_ptr(),
-                                       F16 if out.dtype == torch.float16 else F32, int(standard_domain)))
+        rc = _nat.dequant(hal._addr, w._addr, out, standard_domain, stream)
+        if rc < 0:
+            if out.dtype not in (torch.float16, torch.float32) or not out.is_cuda or not out.is_contiguous():
+                raise QWGemmError(3, "out must be a contiguous CUDA float16/float32 tensor")
+            if out.numel() != w.n * w.k:
+                raise QWGemmError(3, f"out has {out.numel()} elements, expected {w.n * w.k}")
+        _refused(rc, "dequant")
 
     @staticmethod
     def quantize(hal: QWHal, w: torch.Tensor, container: ContainerKind = incumbentHQ4G32,
                  out: Optional[torch.Tensor] = None, stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
         """Load-time quantizer (HQ4Quantizer in Sources/Foundation/QWLoad; Scripts/quantize/hq4.py:54-123):
         f32 [n, k] on the device -> packed blocks, byte-identical to the reference's Python packer."""
+        if out is not None:
+            rc = _nat.quantize(hal._addr, w, container.kind, container.bits, container.group, out, container.block_bytes, stream)
+            if rc == 0:
+                return out
+            if rc > 0:
+                _check(rc)
         if w.dtype != torch.float32 or not w.is_cuda or not w.is_contiguous() or w.dim() != 2:
             raise QWGemmError(3, "w must be a contiguous 2-D CUDA float32 tensor")
         n, k = w.shape

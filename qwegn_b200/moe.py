@@ -10,7 +10,8 @@ import torch
 
 from . import _lib
 from ._lib import F16, F32, WeightViewC
-from .gemm import QWGemmError, QWHal, QWWeightView, _check, _stream_ptr, check_device_tensor
+from . import gemm
+from .gemm import QWGemmError, QWHal, QWWeightView, _check, _refused, _stream_ptr, check_device_tensor
 
 _i32, _i64, _vp, _sz = ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p, ctypes.c_size_t
 _WV = ctypes.POINTER(WeightViewC)
@@ -59,6 +60,12 @@ class QWMoEOperator:
     def encodeResident(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor, scratch: torch.Tensor,
                        x_is_rotated: bool = False, stream: Optional[torch.cuda.Stream] = None) -> None:
         """x f16 [T, H]; logits f32 [T, E]; out f16/f32 [T, H]; scratch uint8 of scratchBytes(T) bytes."""
+        rc = gemm._nat.moe(self.hal._addr, self.hal._index, self.bank_gu._addr, self.bank_dn._addr, self.experts, self.inter, self.top_k,
+                           self.norm_topk, self.routed_scale, x, logits, out, scratch, x_is_rotated, stream)
+        if rc == 0:
+            return
+        if rc > 0:
+            _check(rc)
         check_device_tensor(self.hal, x, "x", torch.float16, contiguous=False)
         check_device_tensor(self.hal, logits, "logits", torch.float32)
         check_device_tensor(self.hal, out, "out", (torch.float16, torch.float32))
@@ -71,10 +78,7 @@ class QWMoEOperator:
             raise QWGemmError(3, "out must be a contiguous [T, H] tensor")
         if x.shape[1] != self.hidden:
             raise QWGemmError(3, f"x has {x.shape[1]} columns, the experts take {self.hidden}")
-        _check(_lib.load().qwc_moe_forward(
-            self.hal.handle, _stream_ptr(stream), ctypes.byref(self.bank_gu.c), ctypes.byref(self.bank_dn.c), self.experts,
-            self.inter, x.data_ptr(), x.shape[0], x.stride(0), int(x_is_rotated), logits.data_ptr(), self.top_k,
-            int(self.norm_topk), float(self.routed_scale), out.data_ptr(), _dt(out), scratch.data_ptr(), scratch.numel()))
+        _refused(rc, "encodeResident")
 
 
 class QWGemmMoE:
@@ -84,6 +88,11 @@ class QWGemmMoE:
     def encodeFnRouterGemm(hal: QWHal, weight: torch.Tensor, x: torch.Tensor, y: torch.Tensor, stream=None) -> None:
         """Router logits y f32 [t, e] = x [t, h] . weight [e, h]^T (QWGemmMoERouter.swift:78-125).  weight: the raw router
         plane, bf16 / f16 / f32, un-rotated; x: plain hidden states, f16 or f32."""
+        rc = gemm._nat.router(hal._addr, weight, x, y, stream)
+        if rc == 0:
+            return
+        if rc > 0:
+            _check(rc)
         dts = {torch.float16: 0, torch.float32: 1, torch.bfloat16: 2}
         if weight.dtype not in dts or x.dtype not in (torch.float16, torch.float32) or y.dtype != torch.float32:
             raise QWGemmError(3, "router GEMM takes bf16/f16/f32 weights, f16/f32 activations and f32 logits")
@@ -93,8 +102,7 @@ class QWGemmMoE:
         e = weight.shape[0]
         if weight.shape[1] != h or tuple(y.shape) != (t, e):
             raise QWGemmError(3, "shape mismatch")
-        _check(_lib.load().qwc_moe_router_gemm(hal.handle, _stream_ptr(stream), x.data_ptr(), dts[x.dtype], x.stride(0), t, h,
-                                               weight.data_ptr(), dts[weight.dtype], e, y.data_ptr()))
+        _refused(rc, "encodeFnRouterGemm")
 
     @staticmethod
     def encodeFnMoeRoute(hal: QWHal, logits: torch.Tensor, top_k: int, idx: torch.Tensor, wts: torch.Tensor,
