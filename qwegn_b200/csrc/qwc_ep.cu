@@ -21,7 +21,7 @@
 #include "qwc_common.cuh"
 
 int qwc_launch_gemm_tc_grouped(const qwc_hal*, cudaStream_t, const qwc_weight_view*, const void*, int64_t, const qwc_moe_tile*,
-                               const int32_t*, int64_t, void*, int, int64_t, int, int);
+                               const int32_t*, int64_t, void*, int, int64_t, int, int, int);
 bool qwc_gemm_tc_supported(const qwc_hal*, const qwc_weight_view*, int64_t, int);
 
 namespace {
@@ -535,8 +535,10 @@ int qwc_ep_experts(qwc_hal* hal, qwc_stream stream, const qwc_ep_ctx* ctx, const
                                 static_cast<int>(h), 1, expert_off_local, tiles_gu, tiles_dn, tile_counts, ret_src, xs, rmax,
                                 static_cast<int>(max_gu), static_cast<int>(max_dn)));
     int rc;
-    if ((rc = qwc_launch_gemm_tc_grouped(hal, st, bank_gu_local, xs, rmax, tiles_gu, tile_counts, max_gu, sc + L.hs, QWC_F16, inter, xrows, gu_epi))) return rc;
-    if ((rc = qwc_launch_gemm_tc_grouped(hal, st, bank_dn_local, sc + L.hs, rmax, tiles_dn, tile_counts + 1, max_dn, sc + L.dn, QWC_F16, h, xrows, QWC_EPI_NONE))) return rc;
+    if ((rc = qwc_launch_gemm_tc_grouped(hal, st, bank_gu_local, xs, rmax, tiles_gu, tile_counts, max_gu, sc + L.hs, QWC_F16, inter, xrows,
+                                         static_cast<int>((2 * inter + 127) / 128), gu_epi))) return rc;
+    if ((rc = qwc_launch_gemm_tc_grouped(hal, st, bank_dn_local, sc + L.hs, rmax, tiles_dn, tile_counts + 1, max_dn, sc + L.dn, QWC_F16, h, xrows,
+                                         static_cast<int>((h + 127) / 128), QWC_EPI_NONE))) return rc;
     QWC_CUDA_TRY(qwc_launch_pdl(qwc_ep_return_kernel, dim3(ep_grid(hal, rmax, 8)), dim3(256), 0, st, reinterpret_cast<const __half*>(sc + L.dn),
                                 static_cast<const int32_t*>(ret_src), static_cast<const int32_t*>(tile_counts + 2),
                                 static_cast<const int32_t*>(peers.counts[ctx->rank]), static_cast<int>(e_local), static_cast<int>(h),

@@ -44,18 +44,24 @@ constexpr int kBM = 128;        // weight rows per tile (UMMA M)
 constexpr int kBK = 64;         // k per operand stage (one 128-byte swizzle atom of f16)
 constexpr int kConvWarps = 16;
 constexpr int kEpiWarps = 4;
-constexpr int kMaxStages = 8;   // operand stages (one decoded weight tile in TMEM + one activation tile in shared memory each)
+constexpr int kMaxAStages = 4;  // stages of decoded weights (tensor memory)
+constexpr int kMaxXStages = 6;  // stages of activations (shared memory)
 constexpr int kTsFirstConvWarp = 4;   // warps 0..2 as above, warp 3 idle so that converter warp c serves quarter c % 4
 constexpr int kTsWarps = kTsFirstConvWarp + kConvWarps + kEpiWarps;
 constexpr int kTsThreads = kTsWarps * 32;
-constexpr int kTsMaxRaw = 8;    // raw (packed weight) stages
+constexpr int kTsMaxRaw = 4;    // raw (packed weight) stages
+constexpr int kXBoxes = 4;      // box heights of the activation copies
 constexpr int kTsBN = 192;      // most tokens per tile (UMMA N)
 
-// Packed geometry of one 64-wide K tile of one row, and K tiles per raw step.
+// Packed bytes of one 64-wide K tile of one row; K tiles per raw step and the row stride of a raw step in shared memory.
+// A raw step spans 512 k (256 k of 8-bit codes), 288 or 320 bytes of a row, plus 16 bytes that make the stride an odd number of
+// 16-byte units, so a quarter warp's 16-byte loads (lane = row) fall in 8 distinct bank groups.  Long rows because the copies pace
+// this kernel by their count of memory requests (~1.35 cycles per request of up to 128 bytes, whatever its size): an 80-byte piece
+// of a row (128 k) is 1.6 requests, a 336-byte piece of four times the weights 3.6.
 template <int FMT> struct TcFmt;
-template <> struct TcFmt<FMT_HQ4_G32_M5> { static constexpr int kTileBytes = 40, kTilesPerRaw = 2; };
-template <> struct TcFmt<FMT_HQ8_G32> { static constexpr int kTileBytes = 72, kTilesPerRaw = 2; };
-template <> struct TcFmt<FMT_HQ4_G64> { static constexpr int kTileBytes = 36, kTilesPerRaw = 4; };
+template <> struct TcFmt<FMT_HQ4_G32_M5> { static constexpr int kTileBytes = 40, kTilesPerRaw = 8, kRowStride = 336; };
+template <> struct TcFmt<FMT_HQ8_G32> { static constexpr int kTileBytes = 72, kTilesPerRaw = 4, kRowStride = 304; };
+template <> struct TcFmt<FMT_HQ4_G64> { static constexpr int kTileBytes = 36, kTilesPerRaw = 8, kRowStride = 304; };
 
 struct TcParams {
     void* y;
@@ -64,14 +70,16 @@ struct TcParams {
     int m, n, k;
     int y_f16;
     int raw_stages;
-    int stages;          // operand stages; a power of two
-    int stage_shift;     // log2(stages): slot of stage j = j & (stages - 1), its use count = j >> stage_shift
+    int a_stages;        // stages of decoded weights
+    int x_stages;        // activation stages
     int kt_per_stage;    // 64-wide K tiles per operand stage: 1 or 2 (a divisor of the K tiles of a raw step)
     int acc_stride;      // TMEM columns per accumulator: 192 or 128; the operand stages start at column 2 * acc_stride
     int x_tile_rows;     // activation rows per tile: 192, 128 or 64
+    int x_box[kXBoxes];  // rows of the activation boxes, tallest first
     int x_slot_bytes;    // bytes of one activation stage: kt_per_stage x x_tile_rows x 128 B
-    int raw_row_bytes;   // packed bytes of one raw step of one row: 80 (HQ4_G32_M5) or 144 (HQ8_G32, HQ4_G64)
-    int m_tiles, n_tiles;
+    int split;           // CTAs (pairs) of a cluster that share one tile, each with its part of K; 1: none
+    int early_weights;   // dense call under the static-weights promise
+    int m_tiles, n_tiles;   // token tiles; weight tiles (1 CTA) or pairs of weight tiles (CTA pairs)
     int epilogue;        // QWC_EPI_NONE, or a SwiGLU epilogue: a tile is then 64 gate rows + the 64 matching up rows
     int up_delta;        // dense SwiGLU mode: row distance gate -> up (= n / 2)
     int xch_bytes;       // shared memory of the gate/up exchange buffer (SwiGLU epilogues)
@@ -80,11 +88,16 @@ struct TcParams {
     const int32_t* tile_count;   // device: number of valid entries of `tiles`
 };
 
+struct TsMaps {
+    CUtensorMap w;            // packed weights: box of 64 rows x one raw step
+    CUtensorMap x[kXBoxes];   // activations: boxes of x_box rows x 64 k
+};
+
 // One unit of work of the kernel: 128 weight rows x up to 192 activation rows.
 struct TileInfo {
     int w_row0;     // first weight row (row coordinate of the weight tensor map)
     int w_row1;     // SwiGLU epilogues: first up row (rows 64..127 of the tile); unused otherwise
-    int w_rows;     // valid weight rows in the tile (<= 128)
+    int w_rows;     // valid weight rows in the tile (<= 128; 0 or less: the second tile of a pair is past the end)
     int x_row0;     // first activation row (row coordinate of the activation tensor map)
     int x_rows;     // valid activation rows
     int y_col0;     // output column of weight row 0 of the tile
@@ -125,12 +138,42 @@ __device__ __forceinline__ uint64_t pack_desc(uint32_t lo, uint32_t hi) {
 
 // kind::f16 instruction descriptor: D = f32, A = B = f16, both K-major, M = 128 weight rows, N = tokens of the
 // tile rounded up to a multiple of 16 (16..256).
-__device__ __forceinline__ uint32_t make_idesc(int n_tokens) {
-    return (1u << 4) | (static_cast<uint32_t>(n_tokens >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
+template <int CG> __device__ __forceinline__ uint32_t make_idesc(int n_tokens) {
+    return (1u << 4) | (static_cast<uint32_t>(n_tokens >> 3) << 17) | (static_cast<uint32_t>(CG * kBM >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// ---- CTA pairs (CG = 2): two CTAs of a cluster run one MMA of 256 weight rows --------------------------------------------
+// Shared-memory address of the same object in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+// No cluster-scope release: what these arrivals publish lives in tensor memory and is ordered by tcgen05.wait /
+// tcgen05.fence (a release at cluster scope cost the converters ~1500 cycles per stage).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// As tma_load_2d, into this CTA's shared memory, counted on a barrier of either CTA of the pair (cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+
+// Arrives on `bar` (CG = 2: on the barrier at this offset of both CTAs of the pair, `mask`) when the MMAs issued so far are done.
+template <int CG> __device__ __forceinline__ void umma_commit(uint64_t* bar, uint16_t mask) {
+    if (CG == 1)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                     "h"(mask)
+                     : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -192,11 +235,37 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, c
     }
 }
 
+// The same for two barriers: both polls are in flight together (a poll of a completed phase takes ~50 cycles, and the MMA
+// warp's turn is a chain).
+__device__ __forceinline__ bool mbar_wait_spin2(uint64_t* bar_a, uint32_t parity_a, uint64_t* bar_b, uint32_t parity_b,
+                                                const volatile int* abort_flag) {
+    uint64_t t0 = 0;
+    for (uint32_t i = 0;; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+            "and.pred p, p, q;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar_a)), "r"(parity_a), "r"(smem_u32(bar_b)), "r"(parity_b)
+            : "memory");
+        if (ok) return true;
+        if ((i & 1023u) == 1023u) {
+            const uint64_t now = qwc_globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            if (*abort_flag || now - t0 > QWC_WAIT_LIMIT_NS) return false;
+        }
+    }
+}
+
 // Tile number `tile` of the launch: from the device-side list (grouped mode) or the dense (weight tile, token tile) grid.
-__device__ __forceinline__ TileInfo tc_get_tile(const TcParams& p, int tile) {
+// CG = 2: the tile of CTA `rank` of pair `tile`; neighbouring weight tiles with the same tokens form a pair.
+template <int CG> __device__ __forceinline__ TileInfo tc_get_tile(const TcParams& p, int tile, int rank) {
     TileInfo t;
     if (p.tiles != nullptr) {
-        const qwc_moe_tile g = p.tiles[tile];
+        const qwc_moe_tile g = p.tiles[CG * tile + rank];
         t.w_row0 = g.w_row0;
         t.w_row1 = g.pad0;
         t.w_rows = g.w_rows;
@@ -204,7 +273,7 @@ __device__ __forceinline__ TileInfo tc_get_tile(const TcParams& p, int tile) {
         t.x_rows = g.x_rows;
         t.y_col0 = g.y_col0;
     } else {
-        const int nt = tile / p.m_tiles, mt = tile % p.m_tiles;   // token tiles fastest: CTAs share weight rows in L2
+        const int nt = CG * (tile / p.m_tiles) + rank, mt = tile % p.m_tiles;   // token tiles fastest: CTAs share weight rows in L2
         if (p.epilogue == QWC_EPI_NONE) {
             t.w_row0 = nt * kBM;
             t.w_row1 = 0;
@@ -212,7 +281,7 @@ __device__ __forceinline__ TileInfo tc_get_tile(const TcParams& p, int tile) {
         } else {
             t.w_row0 = nt * (kBM / 2);
             t.w_row1 = t.w_row0 + p.up_delta;
-            t.w_rows = kBM;
+            t.w_rows = t.w_row0 < p.up_delta ? kBM : 0;
         }
         t.x_row0 = mt * p.x_tile_rows;
         t.x_rows = min(p.x_tile_rows, p.m - t.x_row0);
@@ -284,9 +353,10 @@ __device__ __forceinline__ void tc_swiglu_chunk(const TcParams& p, const TileInf
     const int esz = p.y_f16 ? 2 : 4;
     uint8_t* yrow = static_cast<uint8_t*>(p.y) + (static_cast<int64_t>(ti.x_row0 + tok0) * p.ldy + ti.y_col0 + hrow) * esz;
     const int64_t ystep = p.ldy * esz;
+    const int rows = ti.w_rows > 0 ? ti.x_rows : 0;
 #pragma unroll
     for (int jj = 0; jj < HALF; ++jj) {
-        if (tok0 + jj < ti.x_rows) {
+        if (tok0 + jj < rows) {
             if (p.y_f16) *reinterpret_cast<__half*>(yrow) = __float2half_rn(h[jj]);
             else *reinterpret_cast<float*>(yrow) = __half2float(__float2half_rn(h[jj]));
         }
@@ -362,6 +432,27 @@ __device__ __forceinline__ void tc_epilogue_tile(const TcParams& p, const TileIn
 }
 
 
+// The epilogue of 16 tokens whose sums are in registers already (split K): tokens tok0 .. tok0 + 15 of the tile.
+__device__ __forceinline__ void tc_epilogue_group16(const TcParams& p, const TileInfo& ti, const uint32_t rr[16], uint8_t* xch, int quarter,
+                                                    int lane, int tok0) {
+    if (p.epilogue != QWC_EPI_NONE) {
+        tc_swiglu_chunk<16>(p, ti, rr, xch, quarter >= 2, (quarter & 1) * 32 + lane, lane, tok0);
+        return;
+    }
+    const int wr = quarter * 32 + lane, esz = p.y_f16 ? 2 : 4;
+    if (wr >= ti.w_rows) return;
+    const int64_t ystep = p.ldy * esz;
+    uint8_t* yp = static_cast<uint8_t*>(p.y) + (static_cast<int64_t>(ti.x_row0 + tok0) * p.ldy + ti.y_col0 + wr) * esz;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        if (tok0 + i < ti.x_rows) {
+            if (p.y_f16) *reinterpret_cast<__half*>(yp) = __float2half_rn(__uint_as_float(rr[i]));
+            else *reinterpret_cast<float*>(yp) = __uint_as_float(rr[i]);
+        }
+        yp += ystep;
+    }
+}
+
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t r[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
@@ -375,12 +466,20 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t r[32]) 
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // D[tmem] (+)= A[tmem] * B[smem desc]: M = 128, K = 16, A = 128 lanes x 8 columns of f16 pairs.
+template <int CG>
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if (CG == 1)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
 
 // Decode the 64 k of one K tile of one row, held in registers as packed words, into 32 f16 pairs in natural k order:
@@ -432,70 +531,56 @@ __device__ __forceinline__ void decode_tile_natural(const uint32_t* w, uint32_t*
     }
 }
 
-// The packed words of K tile `sub` of a raw step of one row (src = the row's bytes of the raw step in shared memory).
-// Rows of a raw step are 80 or 144 bytes apart, so a quarter warp's 16-byte loads fall in 8 distinct bank groups.
-template <int FMT>
-__device__ __forceinline__ void load_tile_words(const uint8_t* src, int sub, uint32_t* w) {
-    if (FMT == FMT_HQ4_G32_M5) {
-        // 40 bytes at offset 0 (16-byte aligned) or 40 (8-byte aligned)
-        if (sub == 0) {
-            const uint4 a = *reinterpret_cast<const uint4*>(src), b = *reinterpret_cast<const uint4*>(src + 16);
-            const uint2 d = *reinterpret_cast<const uint2*>(src + 32);
-            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w; w[8] = d.x; w[9] = d.y;
+// The packed words of one K tile of one row: `src` = the two K tiles it is the even or odd one of (80, 144 or 72 bytes, 16- or
+// 8-byte aligned) in shared memory.
+template <int FMT, bool ODD>
+__device__ __forceinline__ void load_tile_words(const uint8_t* src, uint32_t* w) {
+    constexpr int kWords = TcFmt<FMT>::kTileBytes / 4;
+    constexpr int kWide = FMT == FMT_HQ4_G64 ? 2 : 4;   // words of the widest aligned access
+    constexpr int b = ODD ? kWords : 0;                 // first word of the tile inside the pair
+    int i = 0;
+#pragma unroll
+    for (int k = 0; k < kWords; ++k) {
+        if (k < i) continue;
+        const int at = b + k;
+        if (kWide == 4 && at % 4 == 0 && k + 4 <= kWords) {
+            const uint4 v = *reinterpret_cast<const uint4*>(src + 4 * at);
+            w[k] = v.x; w[k + 1] = v.y; w[k + 2] = v.z; w[k + 3] = v.w;
+            i = k + 4;
+        } else if (at % 2 == 0 && k + 2 <= kWords) {
+            const uint2 v = *reinterpret_cast<const uint2*>(src + 4 * at);
+            w[k] = v.x; w[k + 1] = v.y;
+            i = k + 2;
         } else {
-            const uint2 d = *reinterpret_cast<const uint2*>(src + 40);
-            const uint4 a = *reinterpret_cast<const uint4*>(src + 48), b = *reinterpret_cast<const uint4*>(src + 64);
-            w[0] = d.x; w[1] = d.y; w[2] = a.x; w[3] = a.y; w[4] = a.z; w[5] = a.w; w[6] = b.x; w[7] = b.y; w[8] = b.z; w[9] = b.w;
+            w[k] = *reinterpret_cast<const uint32_t*>(src + 4 * at);
+            i = k + 1;
         }
-    } else if (FMT == FMT_HQ8_G32) {
-        // 72 bytes at offset 0 (16-byte aligned) or 72 (8-byte aligned)
-        if (sub == 0) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint4 a = *reinterpret_cast<const uint4*>(src + 16 * i);
-                w[4 * i] = a.x; w[4 * i + 1] = a.y; w[4 * i + 2] = a.z; w[4 * i + 3] = a.w;
-            }
-            const uint2 d = *reinterpret_cast<const uint2*>(src + 64);
-            w[16] = d.x; w[17] = d.y;
-        } else {
-            const uint2 d = *reinterpret_cast<const uint2*>(src + 72);
-            w[0] = d.x; w[1] = d.y;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint4 a = *reinterpret_cast<const uint4*>(src + 80 + 16 * i);
-                w[2 + 4 * i] = a.x; w[3 + 4 * i] = a.y; w[4 + 4 * i] = a.z; w[5 + 4 * i] = a.w;
-            }
-        }
-    } else {
-        // 36 bytes at offset 36 * sub (4-byte aligned)
-        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src + 36 * sub);
-#pragma unroll
-        for (int i = 0; i < 9; ++i) w[i] = s32[i];
     }
 }
 
 // KS = 64-wide K tiles per operand stage: compile-time, because the loops that use it pace the kernel and every instruction
 // in them counts.
-template <int FMT, int KS>
+template <int FMT, int KS, int CG>
 __global__ void __launch_bounds__(kTsThreads, 1)
-qwc_gemm_ts_kernel(const TcParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
-                   const __grid_constant__ CUtensorMap xmap128, const __grid_constant__ CUtensorMap xmap64,
-                   const __grid_constant__ CUtensorMap wmap64) {
+qwc_gemm_ts_kernel(const TcParams p, const __grid_constant__ TsMaps maps) {
     using F = TcFmt<FMT>;
     constexpr int KPR = F::kTilesPerRaw;
     constexpr int kTileWords = F::kTileBytes / 4;
+    constexpr int SPR = KPR / KS;   // operand stages per raw step
     // Let the next kernel of the stream be scheduled as early as its resources allow (it waits for this grid itself).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // layout (1024-byte aligned base): [X tiles][raw stages][barriers][SwiGLU exchange]
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* xt = smem;
-    uint8_t* raw = xt + p.stages * p.x_slot_bytes;
-    const int raw_stage_bytes = ((kBM * p.raw_row_bytes + 127) / 128) * 128;
+    uint8_t* raw = xt + p.x_stages * p.x_slot_bytes;
+    constexpr int raw_stage_bytes = kBM * F::kRowStride;
     uint64_t* bars = reinterpret_cast<uint64_t*>(raw + p.raw_stages * raw_stage_bytes);
-    uint64_t* full = bars;                         // [kMaxStages]  activations landed (tx) + the four quarter warps stored A
-    uint64_t* empty = bars + kMaxStages;           // [kMaxStages]  tcgen05.commit: the MMAs have read both operands of the stage
-    uint64_t* raw_full = bars + 2 * kMaxStages;    // [kTsMaxRaw]
+    uint64_t* full = bars;                         // [kMaxAStages]    the converters have stored A
+    uint64_t* empty = full + kMaxAStages;             // [kMaxAStages]    tcgen05.commit: the MMAs have read A
+    uint64_t* x_full = empty + kMaxAStages;           // [kMaxXStages] activations landed (tx)
+    uint64_t* x_empty = x_full + kMaxXStages;      // [kMaxXStages] tcgen05.commit: the MMAs have read the activations
+    uint64_t* raw_full = x_empty + kMaxXStages;    // [kTsMaxRaw]
     uint64_t* raw_empty = raw_full + kTsMaxRaw;    // [kTsMaxRaw]
     uint64_t* acc_full = raw_empty + kTsMaxRaw;    // [2]
     uint64_t* acc_empty = acc_full + 2;            // [2]
@@ -506,208 +591,294 @@ qwc_gemm_ts_kernel(const TcParams p, const __grid_constant__ CUtensorMap wmap, c
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < p.stages; ++s) {
-            mbar_init(&full[s], 1 + 4);
+        // CG = 2: what the MMAs wait for is counted on the leader's barriers, the peer's converters and copies included
+        for (int s = 0; s < p.a_stages; ++s) {
+            mbar_init(&full[s], 4 * KS * CG);
             mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < p.x_stages; ++s) {
+            mbar_init(&x_full[s], 1);
+            mbar_init(&x_empty[s], 1);
         }
         for (int s = 0; s < p.raw_stages; ++s) {
             mbar_init(&raw_full[s], 1);
-            mbar_init(&raw_empty[s], 4 * KPR / KS);   // every operand stage of the step: four quarter warps
+            mbar_init(&raw_empty[s], kConvWarps);   // every converter warp leaves every step
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], kEpiWarps);
+            mbar_init(&acc_empty[s], kEpiWarps * CG);
         }
         *abort_flag = 0;
         fence_barrier_init();
     }
     if (warp == 1) {
         // 512 columns.  One CTA per SM, so the allocation cannot contend.
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CG == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
-    __syncthreads();
+    const bool clustered = CG == 2 || p.split > 1;
+    uint32_t crank = 0;   // rank in the cluster: pairs are (2 i, 2 i + 1), the split index is crank / CG
+    if (clustered) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
+    const uint32_t leader = crank / CG * CG;
+    const uint16_t pair_mask = static_cast<uint16_t>(3u << leader);
+    if (CG == 1) __syncthreads();   // (a K split of single CTAs first meets after the main loop)
+    else cluster_sync_all();        // the peer's barriers are initialised before anything arrives on them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Everything above needed no global data.  From here on the kernel reads what earlier kernels of the stream wrote
-    // (tile list, activations, possibly the weights) and writes y: wait for the grid before this one.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // (tile list, activations, possibly the weights) and writes y: wait for the grid before this one.  Under the static-weights
+    // promise a dense call's packed rows may be read at once: the weight producer and the converters start while the previous grid
+    // drains, the activation producer (and with it every MMA) and the epilogue wait.
+    const bool waits = !p.early_weights || warp == 0 || warp >= kTsFirstConvWarp + kConvWarps;
+    if (waits) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const int total_tiles = p.tiles != nullptr ? *p.tile_count : p.m_tiles * p.n_tiles;
-    const int ktiles = p.k / kBK;
-    const int raw_steps = ktiles / KPR;
+    // CG = 2: a "tile" is a pair of tiles, one per CTA of the cluster; CTA 0 (the leader) issues the MMAs of both.
+    // split > 1: the cluster shares one tile, CTA (pair) i takes the i-th part of K (dense calls, one tile per cluster).
+    const int rank = static_cast<int>(crank - leader);
+    const int first_tile = static_cast<int>(blockIdx.x) / (CG * p.split), tile_step = static_cast<int>(gridDim.x) / (CG * p.split);
+    const int total_tiles = p.tiles != nullptr ? *p.tile_count / CG : p.m_tiles * p.n_tiles;
+    int kt0 = 0, ktiles = p.k / kBK;   // this CTA's K tiles: whole units of 256 k, 128 k where K is an odd multiple of it
+    if (p.split > 1) {
+        const int unit = p.k % 256 == 0 ? 4 : 2, units = ktiles / unit, part = static_cast<int>(crank) / CG;
+        kt0 = units * part / p.split * unit;
+        ktiles = units * (part + 1) / p.split * unit - kt0;
+    }
+    const int raw_steps = (ktiles + KPR - 1) / KPR;        // the last one may be partly past the end of K (zero filled)
     const int kstages = ktiles / KS;                       // operand stages per tile
     const uint32_t x_sub_bytes = static_cast<uint32_t>(p.x_slot_bytes / KS);   // one 64-wide K tile of the activations inside a stage
     const uint32_t a_col0 = static_cast<uint32_t>(2 * p.acc_stride);
-    const uint32_t smask = static_cast<uint32_t>(p.stages - 1);
     auto fail = [&](int code) {
         if (!*abort_flag) atomicCAS(p.status, 0, code);
         *abort_flag = 1;
     };
 
-    // Operand stage number j of the kernel (all tiles) holds KS consecutive K tiles, uses slot j % stages in phase
-    // (j / stages) & 1 and reads raw step j * KS / KPR, which uses raw slot r % raw_stages in phase (r / raw_stages) & 1.
+    // Operand stage number j of the kernel (all tiles) holds KS consecutive K tiles; its decoded weights use A stage j % 4 in phase
+    // (j / 4) & 1.  Activation and raw stages are rings of their own: (slot, phase) counters on both sides.
     if (warp == 0) {
         // ---------------- TMA producer: rotated activations (one tile per K tile) ----------------
+        // A tile's tokens, rounded up to 16 (pairs: each CTA holds half of the tokens rounded up to 32), arrive in the shortest box
+        // that holds them: rows that no token needs cost as much to move as others.
         if (lane == 0) {
-            uint32_t j = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                const TileInfo ti = tc_get_tile(p, tile);
-                const CUtensorMap* xm = ti.x_rows <= 64 ? &xmap64 : (ti.x_rows <= 128 ? &xmap128 : &xmap);
-                const uint32_t xbytes = (ti.x_rows <= 64 ? 64u : (ti.x_rows <= 128 ? 128u : static_cast<uint32_t>(p.x_tile_rows))) * kBK * 2u;
-                for (int ks = 0; ks < kstages; ++ks, ++j) {
-                    const uint32_t s = j & smask;
-                    const bool got_x = j < static_cast<uint32_t>(p.stages) || mbar_wait_relaxed(&empty[s], ((j >> p.stage_shift) - 1) & 1u, abort_flag);
-                    if (!got_x) {
+            uint32_t slot = 0, phase = 0;
+            bool first = true, ok = true;
+            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+                const TileInfo ti = tc_get_tile<CG>(p, tile, rank);
+                const int own = CG == 1 ? (ti.x_rows + 15) & ~15 : ((ti.x_rows + 31) & ~31) >> 1;
+                const int row0 = ti.x_row0 + rank * own;
+                int box = p.x_box[0];
+                const CUtensorMap* xm = &maps.x[0];
+#pragma unroll
+                for (int i = 1; i < kXBoxes; ++i)
+                    if (p.x_box[i] >= own) {
+                        box = p.x_box[i];
+                        xm = &maps.x[i];
+                    }
+                const uint32_t xbytes = static_cast<uint32_t>(box) * kBK * 2u * KS * CG;
+                for (int ks = 0; ks < kstages; ++ks) {
+                    if (!first && !mbar_wait_relaxed(&x_empty[slot], phase ^ 1u, abort_flag)) {
                         fail(QWC_DEV_WAIT_EMPTY_TIMEOUT);
                         ok = false;
                         break;
                     }
-                    mbar_arrive_expect_tx(&full[s], xbytes * static_cast<uint32_t>(KS));
+                    if (CG == 1 || rank == 0) mbar_arrive_expect_tx(&x_full[slot], xbytes);
+                    const uint32_t bar = CG == 1 ? 0u : cluster_addr(&x_full[slot], leader);
 #pragma unroll
-                    for (int q = 0; q < KS; ++q)
-                        tma_load_2d(xt + s * p.x_slot_bytes + q * x_sub_bytes, xm, (ks * KS + q) * kBK, ti.x_row0, &full[s]);
+                    for (int q = 0; q < KS; ++q) {
+                        uint8_t* dst = xt + slot * p.x_slot_bytes + q * x_sub_bytes;
+                        const int kx = (kt0 + ks * KS + q) * kBK;
+                        if (CG == 1) tma_load_2d(dst, xm, kx, row0, &x_full[slot]);
+                        else tma_load_2d_pair(dst, xm, kx, row0, bar);
+                    }
+                    if (++slot == static_cast<uint32_t>(p.x_stages)) {
+                        slot = 0;
+                        phase ^= 1u;
+                        first = false;
+                    }
+                }
+            }
+            if (CG == 2 && ok) {
+                // the leader's last commits arrive here too: leave only after they have (the slots' last uses, oldest first)
+                for (int q = 0; q < p.x_stages; ++q) {
+                    if (!first || q < static_cast<int>(slot)) {
+                        const uint32_t t = first ? static_cast<uint32_t>(q) : (slot + q) % p.x_stages;
+                        if (!mbar_wait_relaxed(&x_empty[t], t < slot ? phase : phase ^ 1u, abort_flag)) break;
+                    }
                 }
             }
         }
         __syncwarp();
     } else if (warp == 2) {
-        // ---------------- TMA producer: packed weight rows (one raw step = KPR K tiles) ----------------
-        uint32_t r = 0;
-        int ok = 1;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-            if (lane == 0) {
-                const TileInfo ti = tc_get_tile(p, tile);
-                for (int rs = 0; rs < raw_steps; ++rs, ++r) {
-                    const uint32_t s = r % p.raw_stages;
-                    const bool got_w = r < static_cast<uint32_t>(p.raw_stages) || mbar_wait_relaxed(&raw_empty[s], ((r / p.raw_stages) - 1) & 1u, abort_flag);
-                    if (!got_w) {
+        // ---------------- TMA producer: packed weight rows ----------------
+        if (lane == 0) {
+            uint32_t slot = 0, phase = 0;
+            bool first = true, ok = true;   // first: the ring's first turn finds its slots free
+            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+                const TileInfo ti = tc_get_tile<CG>(p, tile, rank);
+                const int w_row1 = p.epilogue == QWC_EPI_NONE ? ti.w_row0 + kBM / 2 : ti.w_row1;
+                for (int rs = 0; rs < raw_steps; ++rs) {
+                    if (!first && !mbar_wait_relaxed(&raw_empty[slot], phase ^ 1u, abort_flag)) {
                         fail(QWC_DEV_WAIT_EMPTY_TIMEOUT);
-                        ok = 0;
+                        ok = false;
                         break;
                     }
-                    mbar_arrive_expect_tx(&raw_full[s], static_cast<uint32_t>(kBM * p.raw_row_bytes));
-                    if (p.epilogue == QWC_EPI_NONE) {
-                        tma_load_2d(raw + s * raw_stage_bytes, &wmap, rs * (p.raw_row_bytes / 8), ti.w_row0, &raw_full[s]);
-                    } else {   // 64 gate rows, then the 64 up rows that pair with them
-                        tma_load_2d(raw + s * raw_stage_bytes, &wmap64, rs * (p.raw_row_bytes / 8), ti.w_row0, &raw_full[s]);
-                        tma_load_2d(raw + s * raw_stage_bytes + (kBM / 2) * p.raw_row_bytes, &wmap64, rs * (p.raw_row_bytes / 8),
-                                    ti.w_row1, &raw_full[s]);
+                    mbar_arrive_expect_tx(&raw_full[slot], static_cast<uint32_t>(raw_stage_bytes));
+                    // two boxes of 64 rows: neighbours, or (SwiGLU epilogues) 64 gate rows and the 64 up rows that pair with them
+                    uint8_t* dst = raw + slot * raw_stage_bytes;
+                    const int wx = (kt0 + rs * KPR) * F::kTileBytes / 8;
+                    tma_load_2d(dst, &maps.w, wx, ti.w_row0, &raw_full[slot]);
+                    tma_load_2d(dst + raw_stage_bytes / 2, &maps.w, wx, w_row1, &raw_full[slot]);
+                    if (++slot == static_cast<uint32_t>(p.raw_stages)) {
+                        slot = 0;
+                        phase ^= 1u;
+                        first = false;
                     }
                 }
             }
-            ok = __shfl_sync(0xFFFFFFFFu, ok, 0);
         }
+        __syncwarp();
     } else if (warp == 1) {
+        if (CG == 1 || rank == 0) {
         // ------------------------------- MMA issuer (whole warp in lockstep, one elected lane issues) ----------------
-        uint32_t j = 0, tiles_done = 0;
+        uint32_t as = 0, a_phase = 0, tiles_done = 0, xs = 0, x_phase = 0;
         bool ok = true;
         const uint64_t b_d0 = umma_desc_sw128(smem_u32(xt));
         const uint32_t b_lo0 = static_cast<uint32_t>(b_d0), b_hi = static_cast<uint32_t>(b_d0 >> 32);
         const uint32_t b_step = static_cast<uint32_t>(p.x_slot_bytes) >> 4;
-        int next_rows = total_tiles > 0 ? tc_get_tile(p, min(static_cast<int>(blockIdx.x), total_tiles - 1)).x_rows : 0;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++tiles_done) {
-            const int as = tiles_done & 1;
-            if (tiles_done >= 2 && !mbar_wait_spin(&acc_empty[as], ((tiles_done >> 1) - 1) & 1, abort_flag)) {
+        int next_rows = total_tiles > 0 ? tc_get_tile<CG>(p, min(first_tile, total_tiles - 1), 0).x_rows : 0;
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++tiles_done) {
+            const int acc = tiles_done & 1;
+            if (tiles_done >= 2 && !mbar_wait_spin(&acc_empty[acc], ((tiles_done >> 1) - 1) & 1, abort_flag)) {
                 if (lane == 0) fail(QWC_DEV_WAIT_TMEM_TIMEOUT);
                 break;
             }
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(as * p.acc_stride);
-            const uint32_t idesc = make_idesc(min(p.acc_stride, (next_rows + 15) & ~15));
+            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * p.acc_stride);
+            const uint32_t idesc = make_idesc<CG>(min(p.acc_stride, (next_rows + (16 * CG - 1)) & ~(16 * CG - 1)));
             {   // the entry of the tile after this one is fetched now: a list entry is a global-memory round trip
-                const int tn = tile + static_cast<int>(gridDim.x);
-                next_rows = tc_get_tile(p, tn < total_tiles ? tn : tile).x_rows;
+                const int tn = tile + tile_step;
+                next_rows = tc_get_tile<CG>(p, tn < total_tiles ? tn : tile, 0).x_rows;
             }
-            for (int ks = 0; ks < kstages; ++ks, ++j) {
-                const uint32_t s = j & smask;
-                const bool got_full = mbar_wait_spin(&full[s], (j >> p.stage_shift) & 1u, abort_flag);   // all lanes poll: measured faster than one polling lane
+            for (int ks = 0; ks < kstages; ++ks) {
+                const bool got_full = mbar_wait_spin2(&full[as], a_phase, &x_full[xs], x_phase, abort_flag);   // all lanes poll: measured faster than one polling lane
                 if (!got_full) {
                     if (lane == 0) fail(QWC_DEV_WAIT_FULL_TIMEOUT);
                     ok = false;
                     break;
                 }
                 tc_fence_after();   // the converters' tcgen05.st happen-before these MMAs
-                const uint32_t b_lo = b_lo0 + s * b_step;
-                const uint32_t a_tmem = tmem_base + a_col0 + s * 32 * KS;
+                const uint32_t b_lo = b_lo0 + xs * b_step;
+                const uint32_t a_tmem = tmem_base + a_col0 + as * (32 * KS);
                 if (elect_one()) {
 #pragma unroll
                     for (int h = 0; h < KS; ++h) {
                         const uint32_t bh = b_lo + h * (x_sub_bytes >> 4);
 #pragma unroll
                         for (int q = 0; q < kBK / 16; ++q)
-                            umma_f16_ts(d_tmem, a_tmem + (h * 4 + q) * 8, pack_desc(bh + 2 * q, b_hi), idesc, (ks > 0 || h > 0 || q > 0) ? 1u : 0u);
+                            umma_f16_ts<CG>(d_tmem, a_tmem + (h * 4 + q) * 8, pack_desc(bh + 2 * q, b_hi), idesc, (ks > 0 || h > 0 || q > 0) ? 1u : 0u);
                     }
-                    umma_commit(&empty[s]);
+                    umma_commit<CG>(&empty[as], pair_mask);
+                    umma_commit<CG>(&x_empty[xs], pair_mask);
                 }
                 __syncwarp();
+                if (++xs == static_cast<uint32_t>(p.x_stages)) {
+                    xs = 0;
+                    x_phase ^= 1u;
+                }
+                if (++as == static_cast<uint32_t>(p.a_stages)) {
+                    as = 0;
+                    a_phase ^= 1u;
+                }
             }
-            if (ok && elect_one()) umma_commit(&acc_full[as]);
+            if (ok && elect_one()) umma_commit<CG>(&acc_full[acc], pair_mask);
             __syncwarp();
+        }
         }
         __syncwarp();
     } else if (warp >= kTsFirstConvWarp && warp < kTsFirstConvWarp + kConvWarps) {
         // ------------------------------- converters -------------------------------
-        // Converter warp c: TMEM lane quarter c & 3, operand stages j with j % 4 == c >> 2.  A thread owns one weight row.
+        // Converter warp c: TMEM lane quarter c & 3, K tile (c >> 2) % KS of the operand stages j with j % NCL == (c >> 2) / KS.  One
+        // tile per stage and warp: between the moment a stage is free and the moment it is filled again there is one store, the
+        // decode came before.  A thread owns one weight row.  Every warp visits every raw step in order, so its parity waits are
+        // exact whatever the stages it finds there.
         const int c = warp - kTsFirstConvWarp;
-        const int qd = c & 3, cl = c >> 2;
-        const uint32_t row_ofs = static_cast<uint32_t>(qd * 32 + lane) * p.raw_row_bytes;
-        const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + a_col0;
+        constexpr uint32_t NCL = 4 / KS;   // classes of stages
+        const int qd = c & 3, half = (c >> 2) % KS, cl = (c >> 2) / KS;
+        const uint32_t row_ofs = static_cast<uint32_t>(qd * 32 + lane) * F::kRowStride;
+        const uint32_t full_leader = CG == 1 ? 0u : cluster_addr(full, leader);
+        const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + a_col0 + half * 32u;
         bool ok = true;
+        uint32_t slot = 0, phase = 0;
         uint32_t jbase = 0;   // operand stages of the tiles already done
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, jbase += kstages) {
-            // first stage of this tile that belongs to this warp's class
-            for (uint32_t j = jbase + ((cl + 4u - (jbase & 3u)) & 3u); j < jbase + kstages; j += 4) {
-                const uint32_t kt0 = j * KS;          // first K tile of the stage (KS divides KPR: one raw step per stage)
-                const uint32_t r = kt0 / KPR;
-                const int sub0 = static_cast<int>(kt0 % KPR);
-                const uint32_t rslot = r % p.raw_stages, rpar = (r / p.raw_stages) & 1u;
-                const uint32_t s = j & smask, use = j >> p.stage_shift;
-                // The parity wait is exact: raw_stages is a power of two, so this warp (every fourth stage) meets every phase
-                // of the raw slots it uses, and it has seen phase k - 1 of a slot complete before it waits for phase k.
-                const bool got_raw = mbar_wait(&raw_full[rslot], rpar, abort_flag);
-                if (!got_raw) {
+        uint32_t as = cl, use = 0;   // A stage of this warp's next operand stage and how often it was filled before (a_stages >= NCL)
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, jbase += kstages) {
+            for (int rs = 0; rs < raw_steps && ok; ++rs) {
+                if (!mbar_wait(&raw_full[slot], phase, abort_flag)) {
                     if (lane == 0) fail(QWC_DEV_WAIT_FULL_TIMEOUT);
                     ok = false;
                     break;
                 }
-                const uint8_t* src = raw + rslot * raw_stage_bytes + row_ofs;
-                uint32_t w[kTileWords];
-                uint32_t a32[32];
-                uint32_t w1[KS == 2 ? kTileWords : 1];
-                load_tile_words<FMT>(src, sub0, w);
-                if (KS == 2) load_tile_words<FMT>(src, sub0 + 1, w1);
-                decode_tile_natural<FMT>(w, a32);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_empty[rslot]);   // the packed words of the stage are in registers
-                // only now wait for the operand stage: the decode above overlapped the MMAs that were reading it
-                const bool got_empty = use == 0 || mbar_wait(&empty[s], (use - 1) & 1u, abort_flag);
-                if (!got_empty) {
-                    if (lane == 0) fail(QWC_DEV_WAIT_EMPTY_TIMEOUT);
-                    ok = false;
-                    break;
+                const uint8_t* src = raw + slot * raw_stage_bytes + row_ofs;
+                // this warp's stages of the step: sub = operand stage inside the step
+                const uint32_t j0 = jbase + static_cast<uint32_t>(rs) * SPR;
+                const int nsub = min(SPR, kstages - rs * SPR);
+                int sub = static_cast<int>((cl + NCL - (j0 % NCL)) % NCL);
+                if (sub >= nsub) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&raw_empty[slot]);   // nothing for this warp here
                 }
-                tc_fence_after();   // the MMAs that read this A stage are complete (tcgen05.commit -> empty[s])
-                tmem_st32(lane_taddr + s * 32 * KS, a32);
-                if (KS == 2) {
-                    tmem_st_wait();   // the first store has read its registers
-                    decode_tile_natural<FMT>(w1, a32);
-                    tmem_st32(lane_taddr + s * 64 + 32, a32);
+                for (; sub < nsub; sub += NCL) {
+                    
+                    uint32_t w[kTileWords];
+                    uint32_t a32[32];
+                    const int t = sub * KS + half;   // K tile of the raw step
+                    const uint8_t* pair = src + (t >> 1) * (2 * F::kTileBytes);
+                    if (t & 1) load_tile_words<FMT, true>(pair, w);
+                    else load_tile_words<FMT, false>(pair, w);
+                    decode_tile_natural<FMT>(w, a32);
+                    if (sub + static_cast<int>(NCL) >= nsub) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&raw_empty[slot]);   // the warp's last packed words of the step are in registers
+                    }
+                    // only now wait for the operand stage: the decode above overlapped the MMAs that were reading it
+                    const bool got_empty = use == 0 || mbar_wait(&empty[as], (use - 1) & 1u, abort_flag);
+                    if (!got_empty) {
+                        if (lane == 0) fail(QWC_DEV_WAIT_EMPTY_TIMEOUT);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();   // the MMAs that read this A stage are complete (tcgen05.commit -> empty[s])
+                    tmem_st32(lane_taddr + as * (32 * KS), a32);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (CG == 1) mbar_arrive(&full[as]);
+                        else mbar_arrive_cluster(full_leader + as * 8u);
+                    }
+                    as += NCL;
+                    if (as >= static_cast<uint32_t>(p.a_stages)) {
+                        as -= p.a_stages;
+                        ++use;
+                    }
                 }
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[s]);
+                if (++slot == static_cast<uint32_t>(p.raw_stages)) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
             }
         }
     } else if (warp >= kTsFirstConvWarp + kConvWarps) {
         // ------------------------------- epilogue -------------------------------
         const int quarter = warp & 3;
         uint32_t tiles_done = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tiles_done) {
-            const TileInfo ti = tc_get_tile(p, tile);
+        for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++tiles_done) {
+            const TileInfo ti = tc_get_tile<CG>(p, tile, rank);
             const int as = tiles_done & 1;
             const bool got = mbar_wait_relaxed(&acc_full[as], (tiles_done >> 1) & 1, abort_flag);
             // The four warps decide together whether to go on: the SwiGLU epilogue meets at a named barrier per 16
@@ -720,18 +891,76 @@ qwc_gemm_ts_kernel(const TcParams p, const __grid_constant__ CUtensorMap wmap, c
                 break;
             }
             tc_fence_after();
+            if (p.split > 1) break;   // the partial sums meet below, when every CTA of the cluster has left its main loop
             tc_epilogue_tile(p, ti, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(as * p.acc_stride), xch,
                              quarter, lane);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[as]);
+            if (lane == 0) {
+                if (CG == 1) mbar_arrive(&acc_empty[as]);
+                else mbar_arrive_cluster(cluster_addr(&acc_empty[as], leader));
+            }
         }
     }
 
+    if (p.split > 1) {
+        // Split K: the 16-token groups of the tile are dealt to the CTAs of the cluster (group g to split index g % split), every
+        // CTA stores its partial sums of the others' groups into their shared memory (their operand rings are idle by now) and
+        // finishes its own: sums in split order, so the result does not depend on timing.
+        const TileInfo ti = tc_get_tile<CG>(p, first_tile, rank);
+        const int groups = (ti.x_rows + 15) / 16, part = static_cast<int>(crank) / CG, split = p.split;
+        const int quarter = warp & 3, own_max = (groups + split - 1) / split;
+        const uint32_t acc0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+        float* buf = reinterpret_cast<float*>(smem) + quarter * 32 + lane;   // [source split index][own group][16 tokens][128 rows]
+        const bool epi = warp >= kTsFirstConvWarp + kConvWarps;
+        tc_fence_before();
+        cluster_sync_all();
+        tc_fence_after();
+        const bool split_ok = *abort_flag == 0;   // nothing writes the flag any more: the same for every warp of the CTA
+        if (epi && split_ok) {   // (sending from the idle converter warps too was no faster)
+            for (int g = 0; g < groups; ++g) {
+                const int to = g % split;
+                if (to == part) continue;
+                uint32_t rr[16];
+                tmem_ld16(acc0 + g * 16, rr);
+                tmem_ld_wait();
+                const uint32_t dst = cluster_addr(buf + ((part * own_max + g / split) * 16) * kBM, static_cast<uint32_t>(to * CG + rank));
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + i * kBM * 4), "r"(rr[i]) : "memory");
+            }
+        }
+        cluster_sync_all();
+        if (epi && split_ok) {
+            for (int g = part; g < groups; g += split) {
+                uint32_t rr[16];
+                tmem_ld16(acc0 + g * 16, rr);
+                tmem_ld_wait();
+                float sum[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sum[i] = 0.0f;
+                for (int from = 0; from < split; ++from) {
+                    const float* src = buf + ((from * own_max + g / split) * 16) * kBM;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[i] += from == part ? __uint_as_float(rr[i]) : src[i * kBM];
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) rr[i] = __float_as_uint(sum[i]);
+                tc_epilogue_group16(p, ti, rr, xch, quarter, lane, g * 16);
+            }
+        }
+    }
+    // After a failed wait copies may still be in flight into this CTA's shared memory: give them time to land (bounded).
+    if (*abort_flag)
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);
     tc_fence_before();
-    __syncthreads();
+    if (CG == 1) __syncthreads();
+    else cluster_sync_all();   // nobody leaves while the peer may still arrive on this CTA's barriers or read its operands
     tc_fence_after();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    if (warp == 1) {
+        if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
 }
 
 // Staging pre-pass of the tensor path: rows of ldx -> rows of ldo, rotated (FWHT-32 per unit) or copied.  Eight elements per
@@ -753,34 +982,57 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-template <int FMT, int KS>
-int launch_ts_inst(const qwc_hal* hal, cudaStream_t st, const TcParams& p, const CUtensorMap& wmap, const CUtensorMap& wmap64,
-                   const CUtensorMap* xmaps, int smem, int grid) {
-    // once per device and instantiation; racing first calls both set the same value, which is harmless
-    static std::atomic<bool> configured[64];
-    if (!configured[hal->device & 63].load(std::memory_order_acquire)) {
-        QWC_CUDA_TRY(cudaFuncSetAttribute(qwc_gemm_ts_kernel<FMT, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        configured[hal->device & 63].store(true, std::memory_order_release);
-    }
+template <int FMT, int KS, int CG>
+int launch_ts_inst(const qwc_hal* hal, cudaStream_t st, const TcParams& p, const TsMaps& maps, int smem, int grid) {
+    if (int rc = qwc_allow_smem<qwc_gemm_ts_kernel<FMT, KS, CG>>(hal, 227 * 1024)) return rc;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kTsThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = CG * p.split;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    QWC_CUDA_TRY(cudaLaunchKernelEx(&cfg, qwc_gemm_ts_kernel<FMT, KS>, p, wmap, xmaps[0], xmaps[1], xmaps[2], wmap64));
+    cfg.numAttrs = CG * p.split == 1 ? 1 : 2;
+    QWC_CUDA_TRY(cudaLaunchKernelEx(&cfg, qwc_gemm_ts_kernel<FMT, KS, CG>, p, maps));
     return QWC_OK;
 }
 
+// Clusters of `size` CTAs (one per SM) that can run at once: asked once per device and size.
+int ts_max_clusters(const qwc_hal* hal, int size) {
+    static std::atomic<int> known[64][9];
+    int n = known[hal->device & 63][size].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (qwc_allow_smem<qwc_gemm_ts_kernel<FMT_HQ4_G32_M5, 4, 1>>(hal, 227 * 1024)) return 0;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(size * hal->sm_count);
+        cfg.blockDim = dim3(kTsThreads);
+        cfg.dynamicSmemBytes = 227 * 1024;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = size;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, qwc_gemm_ts_kernel<FMT_HQ4_G32_M5, 4, 1>, &cfg) != cudaSuccess || n < 1) {
+            (void)cudaGetLastError();
+            n = -1;
+        }
+        known[hal->device & 63][size].store(n, std::memory_order_relaxed);
+    }
+    return n > 0 ? n : 0;
+}
+
 template <int FMT>
-int launch_ts(const qwc_hal* hal, cudaStream_t st, const TcParams& p, const CUtensorMap& wmap, const CUtensorMap& wmap64,
-              const CUtensorMap* xmaps, int smem, int grid) {
-    if (p.kt_per_stage == 2) return launch_ts_inst<FMT, 2>(hal, st, p, wmap, wmap64, xmaps, smem, grid);
-    return launch_ts_inst<FMT, 1>(hal, st, p, wmap, wmap64, xmaps, smem, grid);
+int launch_ts(const qwc_hal* hal, cudaStream_t st, const TcParams& p, int cg, const TsMaps& maps, int smem, int grid) {
+    if (p.kt_per_stage == 2) return cg == 2 ? launch_ts_inst<FMT, 2, 2>(hal, st, p, maps, smem, grid) : launch_ts_inst<FMT, 2, 1>(hal, st, p, maps, smem, grid);
+    return cg == 2 ? launch_ts_inst<FMT, 4, 2>(hal, st, p, maps, smem, grid) : launch_ts_inst<FMT, 4, 1>(hal, st, p, maps, smem, grid);
 }
 
 }  // namespace
@@ -796,7 +1048,7 @@ bool qwc_gemm_tc_supported(const qwc_hal* hal, const qwc_weight_view* w, int64_t
     // wins (N = 17408, K = 5120, us per call, stream / tensor: HQ4_G32 8 tokens 19.0 / 19.1, 9 tokens 22.5 / 18.1; HQ8_G32
     // 4 tokens 25.3 / 33.5 (with so few activation rows the activation reads of all CTAs land on the same few lines, whatever
     // the row stride), 8 tokens 27.8 / 23.2; HQ4_G64 8 tokens 21.7 / 22.7, 9 tokens 23.7 / 22.7)
-    if (w->k % (fmt == FMT_HQ4_G64 ? 256 : 128) != 0 || m < tune_env("QWC_TC_MIN_M", qwc_tc_min_tokens(fmt))) return false;
+    if (w->k % (fmt == FMT_HQ4_G64 ? 256 : 128) != 0 || m < tune_env("QWC_TC_MIN_M", qwc_tc_min_tokens(fmt, w->k))) return false;
     if (reinterpret_cast<uintptr_t>(w->blocks) % 16 != 0) return false;
     return tune_env("QWC_NO_TCGEN05", 0) == 0;
 }
@@ -817,10 +1069,51 @@ size_t qwc_gemm_tc_workspace_bytes(const qwc_weight_view* w, int64_t m, int x_is
     return tc_stages_x(m, x_is_rotated) ? static_cast<size_t>(m) * static_cast<size_t>(tc_stage_ld(w->k, m)) * 2 : 0;
 }
 
+// How a dense call is cut: CTAs per MMA, token rows per tile, CTAs (pairs) that share a tile's K.
+struct TsPlan {
+    int cg, rows, split;
+};
+
+// Cycles of one 128-k step of a tile by its token rows, fitted on CTA pairs (2048 x 8192, 200 tokens: 564, 591, 617, 730 and 864
+// at 64, 96, 128, 160 and 192 rows): up to ~100 rows the MMA warp's turn sets them, from there on the MMAs do.
+static int64_t ts_step_cycles(int rows) { return rows <= 64 ? 554 : (rows <= 128 ? 490 + rows : 618 + (rows - 128) * 38 / 10); }
+
+// Up to 64 tokens a tile is one CTA's (a pair would pad the MMA to 32 tokens per CTA and halve the tiles: 17408 x 5120, 16 tokens
+// 16.0 us against 18.0); above, pairs share the activation tile.  Among tile heights and K splits the plan takes the one whose
+// waves of tiles cost least; a split pays for two meetings of its cluster and the exchange of the partial sums (2.5 us at 16 tokens,
+// 3.5 us at 64, 4.3 us between pairs) and only fills SMs that would idle, so it is considered where all its tiles run at once.
+static TsPlan ts_plan(const qwc_hal* hal, int64_t m, int64_t n_tiles, int64_t k) {
+    TsPlan best{m > 64 ? 2 : 1, 64, 1};
+    if (const int e = tune_env("QWC_TC_CG", 0)) best.cg = e;
+    const int cg = best.cg, env_rows = tune_env("QWC_TC_ROWS", 0), env_split = tune_env("QWC_TC_SPLIT", 0);
+    const int64_t units_n = (n_tiles + cg - 1) / cg, k_units = k % 256 == 0 ? k / 256 : k / 128;
+    int64_t best_cost = INT64_MAX;
+    for (int rows = cg == 1 ? 64 : 32; rows <= (cg == 1 ? 64 : kTsBN); rows += 32) {
+        if (env_rows && cg == 2 && rows != env_rows) continue;
+        const int64_t tiles = units_n * ((m + rows - 1) / rows);
+        for (int split = 1; split * cg <= 8 && split <= k_units; ++split) {
+            if (env_split && split != env_split) continue;
+            if (split == 5 || split == 7) continue;   // cluster sizes that pack badly into the GPCs
+            const int64_t slots = split == 1 ? hal->sm_count / cg : ts_max_clusters(hal, cg * split);
+            if (slots < 1 || (split > 1 && tiles > slots)) continue;
+            const int64_t waves = (tiles + slots - 1) / slots;
+            const int64_t steps = (k_units + split - 1) / split * (k % 256 == 0 ? 2 : 1);
+            const int64_t cost = waves * steps * ts_step_cycles(rows) + (split == 1 ? 0 : (cg == 2 ? 8000 : 4000 + 40 * m));
+            if (cost < best_cost || (cost == best_cost && split == 1)) {
+                best_cost = cost;
+                best.rows = rows;
+                best.split = split;
+            }
+        }
+    }
+    return best;
+}
+
 // Shared by the dense door and the grouped (MoE) door: tensor maps, shared-memory budget, launch.
+// w_tiles: weight tiles per token tile of a grouped call's list (even: neighbouring entries form the tiles of a CTA pair).
 static int tc_run(const qwc_hal* hal, cudaStream_t st, const qwc_weight_view* w, const __half* xr, int64_t ldxr, int64_t m,
                   void* y, int y_dtype, int64_t ldy, const qwc_moe_tile* tiles, const int32_t* tile_count, int64_t max_tiles,
-                  int x_tile_rows, int epilogue) {
+                  int x_tile_rows, int w_tiles, int epilogue) {
     const int fmt = qwc_fmt_of(*w);
     TcParams p{};
     p.tiles = tiles;
@@ -828,65 +1121,83 @@ static int tc_run(const qwc_hal* hal, cudaStream_t st, const qwc_weight_view* w,
     p.y = y;
     p.ldy = ldy;
     p.status = hal->status;
+    p.early_weights = hal->static_weights && tiles == nullptr && !tune_env("QWC_TC_LATE", 0);
     p.m = static_cast<int>(m);
     p.n = static_cast<int>(w->n);
     p.k = static_cast<int>(w->k);
     p.y_f16 = y_dtype == QWC_F16;
-    p.raw_row_bytes = fmt == FMT_HQ4_G32_M5 ? 80 : 144;
-    if (tiles == nullptr) x_tile_rows = m <= 64 ? 64 : (m <= 128 ? 128 : kTsBN);   // dense: the narrowest tile that holds all tokens
+    const int raw_stride = fmt == FMT_HQ4_G32_M5 ? TcFmt<FMT_HQ4_G32_M5>::kRowStride
+                                                 : (fmt == FMT_HQ8_G32 ? TcFmt<FMT_HQ8_G32>::kRowStride : TcFmt<FMT_HQ4_G64>::kRowStride);
+    const int64_t n_tiles1 = epilogue == QWC_EPI_NONE ? (w->n + kBM - 1) / kBM : w->n / kBM;
+    int cg;
+    p.split = 1;
+    if (tiles == nullptr) {
+        const TsPlan plan = ts_plan(hal, m, n_tiles1, w->k);
+        cg = plan.cg;
+        x_tile_rows = plan.rows;
+        p.split = plan.split;
+    } else {
+        cg = w_tiles > 0 && w_tiles % 2 == 0 ? tune_env("QWC_MOE_CG", 2) : 1;
+    }
     if (x_tile_rows > kTsBN) x_tile_rows = kTsBN;
     p.x_tile_rows = x_tile_rows;
-    // Four operand stages.  The issue loop of the MMA warp costs a fixed ~0.2 us per stage (barrier wait, fence, commit), so a
-    // stage of one 64-wide K tile paces the kernel whenever its MMAs are shorter than that: tiles of up to 128 tokens (expert
-    // tiles, verify-sized calls) take 128 k per stage and narrower accumulators to make room in tensor memory.
-    p.kt_per_stage = x_tile_rows <= 128 ? 2 : 1;
-    if (const int ks_env = tune_env("QWC_TC_KS", 0); ks_env == 1 || (ks_env == 2 && x_tile_rows <= 128)) p.kt_per_stage = ks_env;
-    p.stages = 4;
-    if (p.kt_per_stage == 1 && x_tile_rows <= 128 && tune_env("QWC_TC_STAGES", 8) == 8) p.stages = kMaxStages;
-    p.acc_stride = x_tile_rows <= 128 ? 128 : kTsBN;
-    p.stage_shift = p.stages == kMaxStages ? 3 : 2;
+    // Operand stages.  The MMA warp's turn per stage costs ~340 cycles of its own (two barrier waits, fence, election, commits)
+    // next to ~27 per MMA it issues, so a stage holds as many K tiles as leave two stages in tensor memory: tiles of up to 128 tokens
+    // four (16 MMAs of at least ~50 cycles), taller ones two (8 MMAs of 96 cycles).
+    p.acc_stride = x_tile_rows <= 64 ? 64 : (x_tile_rows <= 128 ? 128 : kTsBN);
+    p.kt_per_stage = x_tile_rows <= 128 && w->k % 256 == 0 ? 4 : 2;
+    if (tune_env("QWC_TC_KS", 0) == 2) p.kt_per_stage = 2;
+    p.a_stages = (512 - 2 * p.acc_stride) / (32 * p.kt_per_stage);
+    if (p.a_stages > kMaxAStages) p.a_stages = kMaxAStages;
     p.m_tiles = static_cast<int>((m + x_tile_rows - 1) / x_tile_rows);
     p.epilogue = epilogue;
     p.up_delta = static_cast<int>(w->n / 2);
     p.xch_bytes = epilogue == QWC_EPI_NONE ? 0 : (kBM / 2) * 32 * 2;   // 64 rows x 16 parked tokens (f16) per side
-    p.n_tiles = epilogue == QWC_EPI_NONE ? static_cast<int>((w->n + kBM - 1) / kBM) : static_cast<int>(w->n / kBM);
-    const int raw_stage_bytes = ((kBM * p.raw_row_bytes + 127) / 128) * 128;
-    p.x_slot_bytes = p.kt_per_stage * x_tile_rows * kBK * 2;
-    p.raw_stages = kTsMaxRaw;
-    auto smem_need = [&](int rs) { return 1024 + p.stages * p.x_slot_bytes + rs * raw_stage_bytes + 512 + p.xch_bytes; };
-    while (smem_need(p.raw_stages) > 227 * 1024 && p.raw_stages > 2) p.raw_stages >>= 1;   // a power of two (see the converters' raw wait)
-    if (smem_need(p.raw_stages) > 227 * 1024) return qwc_fail(QWC_ERR_BAD_GEOMETRY, "shared-memory budget exceeded");
-    const int smem = smem_need(p.raw_stages);
+    p.n_tiles = static_cast<int>((n_tiles1 + cg - 1) / cg);
+    const int raw_stage_bytes = kBM * raw_stride;
+    p.x_slot_bytes = p.kt_per_stage * (x_tile_rows / cg) * kBK * 2;
+    // Shared memory: two raw steps; activation stages that span at least 512 k beyond the one in use (they cover the latency of the
+    // copies), then more raw steps.
+    auto smem_need = [&](int rs, int xst) { return 1024 + xst * p.x_slot_bytes + rs * raw_stage_bytes + 512 + p.xch_bytes; };
+    p.raw_stages = 2;
+    p.x_stages = 2;
+    if (smem_need(p.raw_stages, p.x_stages) > 227 * 1024) return qwc_fail(QWC_ERR_BAD_GEOMETRY, "shared-memory budget exceeded");
+    const int want_x = tune_env("QWC_TC_XST", p.kt_per_stage == 4 ? 3 : 5), want_raw = tune_env("QWC_TC_RAW", kTsMaxRaw);
+    while (p.x_stages < want_x && smem_need(p.raw_stages, p.x_stages + 1) <= 227 * 1024) ++p.x_stages;
+    while (p.raw_stages < want_raw && smem_need(p.raw_stages + 1, p.x_stages) <= 227 * 1024) ++p.raw_stages;
+    const int smem = smem_need(p.raw_stages, p.x_stages);
 
     const EncodeFn enc = reinterpret_cast<EncodeFn>(hal->encode_tiled);
-    alignas(64) CUtensorMap wmaps[2];   // packed-weight boxes of 128 rows and (SwiGLU epilogues) 64 rows
-    alignas(64) CUtensorMap xmaps[3];   // activation boxes of x_tile_rows, 128 and 64 rows
+    alignas(64) TsMaps maps;
     const int64_t row_bytes = (w->k / w->group) * qwc_block_bytes(w->kind, w->bits, w->group);
-    for (int i = 0; i < 2; ++i) {
+    const cuuint32_t estr[2] = {1, 1};
+    {
         const cuuint64_t gdim[2] = {static_cast<cuuint64_t>(row_bytes / 8), static_cast<cuuint64_t>(w->n)};
         const cuuint64_t gstride[1] = {static_cast<cuuint64_t>(row_bytes)};
-        cuuint32_t box[2] = {static_cast<cuuint32_t>(p.raw_row_bytes / 8), static_cast<cuuint32_t>(i == 0 ? kBM : kBM / 2)};
-        const cuuint32_t estr[2] = {1, 1};
-        const CUresult cr = enc(&wmaps[i], CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(w->blocks), gdim, gstride, box, estr,
+        const cuuint32_t box[2] = {static_cast<cuuint32_t>(raw_stride / 8), static_cast<cuuint32_t>(kBM / 2)};
+        const CUresult cr = enc(&maps.w, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(w->blocks), gdim, gstride, box, estr,
                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) return qwc_fail(QWC_ERR_CUDA, "cuTensorMapEncodeTiled(weights) failed with %d", static_cast<int>(cr));
     }
-    for (int i = 0; i < 3; ++i) {
+    // box heights: all rows of a tile (a CTA's half of them), then three, two and one quarters where those are multiples of 16
+    const int x_rows = x_tile_rows / cg;
+    for (int i = 0; i < kXBoxes; ++i) {
+        p.x_box[i] = ((x_rows * (kXBoxes - i) / kXBoxes) + 15) / 16 * 16;
         const cuuint64_t gdim[2] = {static_cast<cuuint64_t>(w->k), static_cast<cuuint64_t>(m)};
         const cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ldxr * 2)};
-        const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBK), static_cast<cuuint32_t>(i == 0 ? x_tile_rows : (i == 1 ? 128 : 64))};
-        const cuuint32_t estr[2] = {1, 1};
-        const CUresult cr = enc(&xmaps[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(xr), gdim, gstride, box, estr,
+        const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBK), static_cast<cuuint32_t>(p.x_box[i])};
+        const CUresult cr = enc(&maps.x[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(xr), gdim, gstride, box, estr,
                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) return qwc_fail(QWC_ERR_CUDA, "cuTensorMapEncodeTiled(activations) failed with %d", static_cast<int>(cr));
     }
-    const int64_t ntiles = tiles != nullptr ? max_tiles : static_cast<int64_t>(p.m_tiles) * p.n_tiles;
-    const int grid = static_cast<int>(ntiles < hal->sm_count ? (ntiles < 1 ? 1 : ntiles) : hal->sm_count);
-    if (fmt == FMT_HQ4_G32_M5) return launch_ts<FMT_HQ4_G32_M5>(hal, st, p, wmaps[0], wmaps[1], xmaps, smem, grid);
-    if (fmt == FMT_HQ8_G32) return launch_ts<FMT_HQ8_G32>(hal, st, p, wmaps[0], wmaps[1], xmaps, smem, grid);
-    return launch_ts<FMT_HQ4_G64>(hal, st, p, wmaps[0], wmaps[1], xmaps, smem, grid);
+    const int64_t ntiles = tiles != nullptr ? max_tiles / cg : static_cast<int64_t>(p.m_tiles) * p.n_tiles;
+    const int64_t slots = hal->sm_count / cg;
+    const int grid = p.split > 1 ? cg * p.split * static_cast<int>(ntiles) : cg * static_cast<int>(ntiles < slots ? (ntiles < 1 ? 1 : ntiles) : slots);
+    if (fmt == FMT_HQ4_G32_M5) return launch_ts<FMT_HQ4_G32_M5>(hal, st, p, cg, maps, smem, grid);
+    if (fmt == FMT_HQ8_G32) return launch_ts<FMT_HQ8_G32>(hal, st, p, cg, maps, smem, grid);
+    return launch_ts<FMT_HQ4_G64>(hal, st, p, cg, maps, smem, grid);
 }
 
 // Validation shared with the callers that must refuse before their first launch.
@@ -921,13 +1232,13 @@ int qwc_launch_gemm_tc(const qwc_hal* hal, cudaStream_t st, const qwc_weight_vie
         }
         xr = static_cast<const __half*>(workspace);
     }
-    return tc_run(hal, st, w, xr, ldxr, m, y, y_dtype, ldy, nullptr, nullptr, 0, kTsBN, epilogue);
+    return tc_run(hal, st, w, xr, ldxr, m, y, y_dtype, ldy, nullptr, nullptr, 0, kTsBN, 0, epilogue);
 }
 
 // Grouped expert GEMM: the same kernel over a device-side tile list (see qwc_moe_group_pairs).
 int qwc_launch_gemm_tc_grouped(const qwc_hal* hal, cudaStream_t st, const qwc_weight_view* bank, const void* xs, int64_t pairs,
                                const qwc_moe_tile* tiles, const int32_t* tile_count, int64_t max_tiles, void* y, int y_dtype,
-                               int64_t ldy, int x_tile_rows, int epilogue) {
+                               int64_t ldy, int x_tile_rows, int w_tiles, int epilogue) {
     return tc_run(hal, st, bank, static_cast<const __half*>(xs), bank->k, pairs, y, y_dtype, ldy, tiles, tile_count, max_tiles,
-                  x_tile_rows, epilogue);
+                  x_tile_rows, w_tiles, epilogue);
 }

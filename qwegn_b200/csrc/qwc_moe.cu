@@ -11,7 +11,7 @@
 #include "qwc_common.cuh"
 
 int qwc_launch_gemm_tc_grouped(const qwc_hal*, cudaStream_t, const qwc_weight_view*, const void*, int64_t, const qwc_moe_tile*,
-                               const int32_t*, int64_t, void*, int, int64_t, int, int);
+                               const int32_t*, int64_t, void*, int, int64_t, int, int, int);
 bool qwc_gemm_tc_supported(const qwc_hal*, const qwc_weight_view*, int64_t, int);
 int qwc_launch_gemv_segments(const qwc_hal*, cudaStream_t, const qwc_weight_view*, const void*, int64_t, void*, int, int64_t, int,
                              int64_t, int, const void*, const int32_t*, int64_t);
@@ -794,9 +794,10 @@ static int moe_gather_impl(qwc_hal* hal, qwc_stream stream, const void* x_f16, i
     return QWC_OK;
 }
 
-int qwc_moe_grouped_gemm(qwc_hal* hal, qwc_stream stream, const qwc_weight_view* bank, const void* xs_f16, int64_t pairs,
-                         const qwc_moe_tile* tiles, const int32_t* tile_count, int64_t max_tiles, int32_t x_tile_rows, void* y,
-                         int32_t y_dtype, int64_t ldy, int32_t epilogue) {
+// w_tiles: weight tiles per token tile of the list (what the caller that made the list knows; 0: unknown).
+static int moe_grouped_gemm_impl(qwc_hal* hal, qwc_stream stream, const qwc_weight_view* bank, const void* xs_f16, int64_t pairs,
+                                 const qwc_moe_tile* tiles, const int32_t* tile_count, int64_t max_tiles, int32_t x_tile_rows, void* y,
+                                 int32_t y_dtype, int64_t ldy, int32_t epilogue, int w_tiles) {
     qwc_clear_error();
     if (epilogue < QWC_EPI_NONE || epilogue > QWC_EPI_SILU_PAIR_FWHT) return qwc_fail(QWC_ERR_BAD_SHAPE, "unknown epilogue %d", epilogue);
     if (x_tile_rows != 64 && x_tile_rows != 128 && x_tile_rows != 192 && x_tile_rows != 256)
@@ -812,7 +813,13 @@ int qwc_moe_grouped_gemm(qwc_hal* hal, qwc_stream stream, const qwc_weight_view*
         return qwc_fail(QWC_ERR_BLOCKED, "grouped expert GEMM needs an HQ4_G32_M5 / HQ8_G32 bank with k %% 128 == 0 or an HQ4_G64 bank with k %% 256 == 0, 16-byte aligned");
     if (reinterpret_cast<uintptr_t>(xs_f16) % 16 != 0) return qwc_fail(QWC_ERR_BAD_SHAPE, "xs must be 16-byte aligned");
     return qwc_launch_gemm_tc_grouped(hal, static_cast<cudaStream_t>(stream), bank, xs_f16, pairs, tiles, tile_count, max_tiles, y,
-                                      y_dtype, ldy, x_tile_rows, epilogue);
+                                      y_dtype, ldy, x_tile_rows, w_tiles, epilogue);
+}
+
+int qwc_moe_grouped_gemm(qwc_hal* hal, qwc_stream stream, const qwc_weight_view* bank, const void* xs_f16, int64_t pairs,
+                         const qwc_moe_tile* tiles, const int32_t* tile_count, int64_t max_tiles, int32_t x_tile_rows, void* y,
+                         int32_t y_dtype, int64_t ldy, int32_t epilogue) {
+    return moe_grouped_gemm_impl(hal, stream, bank, xs_f16, pairs, tiles, tile_count, max_tiles, x_tile_rows, y, y_dtype, ldy, epilogue, 0);
 }
 
 int qwc_moe_silu_mul(qwc_hal* hal, qwc_stream stream, const void* gu_f16, int64_t rows, int64_t inter, int32_t rotate,
@@ -970,16 +977,17 @@ int qwc_moe_forward(qwc_hal* hal, qwc_stream stream, const qwc_weight_view* bank
         return rc;
     }
     const int32_t xrows = qwc_moe_tile_rows(pairs, e);
+    const int gu_tiles = static_cast<int>((2 * inter + kTileW - 1) / kTileW), dn_tiles = static_cast<int>((h + kTileW - 1) / kTileW);
     if (gu_epi != QWC_EPI_NONE) {
-        if ((rc = qwc_moe_grouped_gemm(hal, stream, bank_gu, sc + L.xs, pairs, tiles_gu, tile_counts, qwc_moe_max_tiles(pairs, e, 2 * inter),
-                                       xrows, sc + L.hs, QWC_F16, inter, gu_epi))) return rc;
+        if ((rc = moe_grouped_gemm_impl(hal, stream, bank_gu, sc + L.xs, pairs, tiles_gu, tile_counts, qwc_moe_max_tiles(pairs, e, 2 * inter),
+                                       xrows, sc + L.hs, QWC_F16, inter, gu_epi, gu_tiles))) return rc;
     } else {
-        if ((rc = qwc_moe_grouped_gemm(hal, stream, bank_gu, sc + L.xs, pairs, tiles_gu, tile_counts, qwc_moe_max_tiles(pairs, e, 2 * inter),
-                                       xrows, sc + L.gu, QWC_F16, 2 * inter, QWC_EPI_NONE))) return rc;
+        if ((rc = moe_grouped_gemm_impl(hal, stream, bank_gu, sc + L.xs, pairs, tiles_gu, tile_counts, qwc_moe_max_tiles(pairs, e, 2 * inter),
+                                       xrows, sc + L.gu, QWC_F16, 2 * inter, QWC_EPI_NONE, gu_tiles))) return rc;
         if ((rc = qwc_moe_silu_mul(hal, stream, sc + L.gu, pairs, inter, 1, sc + L.hs))) return rc;
     }
-    if ((rc = qwc_moe_grouped_gemm(hal, stream, bank_dn, sc + L.hs, pairs, tiles_dn, tile_counts + 1, qwc_moe_max_tiles(pairs, e, h),
-                                   xrows, sc + L.dn, QWC_F16, h, QWC_EPI_NONE))) return rc;
+    if ((rc = moe_grouped_gemm_impl(hal, stream, bank_dn, sc + L.hs, pairs, tiles_dn, tile_counts + 1, qwc_moe_max_tiles(pairs, e, h),
+                                   xrows, sc + L.dn, QWC_F16, h, QWC_EPI_NONE, dn_tiles))) return rc;
     return qwc_moe_combine(hal, stream, sc + L.dn, QWC_F16, inv_perm, wts, t, k, h, out, out_dtype);
 }
 

@@ -75,6 +75,49 @@ def test_prefill_fused_swiglu_epilogues(hal, oracle, name, shape):
     assert hal.device_status() == 0
 
 
+# Edges of the tensor path's tiling: 64 | 65 tokens between single CTAs and CTA pairs, the heights of a pair's tiles, an odd count of
+# 128-row weight tiles (the last pair's second tile is empty), K in whole and partial packed-weight steps and in odd multiples of
+# 128 (two K tiles per stage instead of four), K split over the CTAs of a cluster (few weight tiles, long K) with uneven parts, and
+# a few tokens whose activations exceed the streaming kernel's shared memory.
+@pytest.mark.parametrize("name", ["HQ4_G32", "HQ8_G32", "HQ4_G64"])
+@pytest.mark.parametrize("m,n,k", [(64, 392, 512), (65, 392, 512), (97, 140, 768), (128, 300, 1280), (161, 130, 512), (193, 640, 256),
+                                   (385, 1100, 1024), (70, 384, 128), (70, 200, 384), (33, 200, 896), (9, 128, 4096), (16, 300, 5120),
+                                   (64, 256, 2816), (100, 128, 7168), (200, 260, 3328), (5, 300, 17408), (3, 64, 28672)])
+def test_tiling_edges(hal, oracle, name, m, n, k):
+    import qwegn_b200 as q
+    if not _tensor_path(name, k):
+        pytest.skip("HQ4_G64 takes the tensor path at K % 256 == 0")
+    assert q.QWGemm.plan(m, n, k, q.CONTAINERS[name]).backend == 2
+    fmt = oracle.FORMATS[name]
+    rng = np.random.default_rng(m + n + k)
+    blocks = oracle.quantize(rng.normal(0.0, 0.02, (n, k)).astype(np.float32), fmt)
+    x = rng.standard_normal((m, k)).astype(np.float16)
+    view = _bank(q, blocks, name)
+    yref = oracle.matmul(blocks, fmt, x)
+    first = _run(q, hal, view, x, out_dtype=torch.float32)
+    assert_matmul_close(first, yref)
+    assert np.array_equal(first, _run(q, hal, view, x, out_dtype=torch.float32))   # the split sums are ordered
+    assert_matmul_close(_run(q, hal, view, oracle.fwht32_f16(x), rotated=True), yref, tight=3e-3)
+    assert hal.device_status() == 0
+
+
+# The paired epilogue over the same edges: 64-row halves whose count is odd (an empty second tile in the last pair) and a split K.
+@pytest.mark.parametrize("m,inter,k", [(70, 192, 512), (200, 64, 1024), (16, 64, 4096), (48, 320, 2560), (150, 128, 7168)])
+def test_tiling_edges_swiglu(hal, oracle, m, inter, k):
+    import qwegn_b200 as q
+    rng = np.random.default_rng(m + inter + k)
+    blocks = oracle.quantize(rng.normal(0.0, 0.03, (2 * inter, k)).astype(np.float32), oracle.HQ4_G32)
+    x = rng.standard_normal((m, k)).astype(np.float16)
+    view = _bank(q, blocks, "HQ4_G32")
+    href = oracle.swiglu_f16(oracle.matmul(blocks, oracle.HQ4_G32, x), rotate=True).astype(np.float32)
+    y = torch.full((m + 1, inter), 7.0, dtype=torch.float16, device="cuda")
+    ws = torch.empty(q.QWGemm.workspaceBytes(hal, view, m, q.EPI_SILU_PAIR_FWHT, False), dtype=torch.uint8, device="cuda")
+    q.QWGemm.encode(hal, view, torch.from_numpy(x).cuda(), y[:m], epi=q.EPI_SILU_PAIR_FWHT, workspace=ws)
+    assert_matmul_close(y[:m].float().cpu().numpy(), href, tight=5e-3)   # as test_prefill_fused_swiglu_epilogues
+    assert (y[m] == 7.0).all()
+    assert hal.device_status() == 0
+
+
 def test_prefill_matches_the_gemv_path_row_by_row(hal, oracle):
     # Twin test (Tests/QWGEMMTests/QWBatchedGemmTests.swift:37-140: batched GEMM vs per-row GEMV, max |d| < 0.05).
     import qwegn_b200 as q
