@@ -32,25 +32,25 @@ inline int moe_tile_rows(int64_t pairs, int64_t e) {
 
 __device__ __forceinline__ bool finite_bits(float v) { return (__float_as_uint(v) & 0x7F800000u) != 0x7F800000u; }
 
-// One warp routes one token.  Lane l holds experts l, l + 32, ... (e <= 512 -> at most 16 per lane).
-__global__ void __launch_bounds__(128) qwc_moe_route_kernel(const float* __restrict__ logits, int t_rows, int e, int k,
-                                                            int norm_topk, float routed_scale, int32_t* __restrict__ idx,
-                                                            float* __restrict__ wts) {
-    pdl_enter();
-    const int lane = threadIdx.x & 31;
-    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (t >= t_rows) return;
-    constexpr int kMaxPer = 16;
-    float pv[kMaxPer];
-    bool valid[kMaxPer];
-    const int per = (e + 31) / 32;
+// One warp routes one token.  Lane l holds experts l, l + 32, ...: PER of them (e <= 32 * PER).  PER is a template argument so
+// that the slices' loads, exponentials, sums and comparisons are independent instructions; with a run-time slice count they
+// ran as one dependent chain (2048 tokens, 256 experts: block 299 -> 296 us).  Lane r < k returns the r-th choice (-1: none)
+// and its weight.
+template <int PER>
+__device__ __forceinline__ void moe_route_token(const float* __restrict__ row, int e, int k, int norm_topk, float routed_scale, int lane,
+                                                int& out_i, float& out_w) {
+    float pv[PER];
+    bool valid[PER];
     float mx = -3.4e38f;
     bool any = false;
 #pragma unroll
-    for (int j = 0; j < kMaxPer; ++j) {
+    for (int j = 0; j < PER; ++j) {
         const int id = lane + 32 * j;
-        pv[j] = (j < per && id < e) ? logits[static_cast<int64_t>(t) * e + id] : 0.0f;
-        valid[j] = j < per && id < e && finite_bits(pv[j]);
+        pv[j] = id < e ? row[id] : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        valid[j] = lane + 32 * j < e && finite_bits(pv[j]);
         if (valid[j]) {
             mx = any ? fmaxf(mx, pv[j]) : pv[j];
             any = true;
@@ -61,63 +61,73 @@ __global__ void __launch_bounds__(128) qwc_moe_route_kernel(const float* __restr
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) wmx = fmaxf(wmx, __shfl_xor_sync(0xFFFFFFFFu, wmx, o));
     const float max_logit = any_finite ? wmx : 0.0f;
-    // total = sum over experts in index order groups (lane-major partial sums, then a warp sum): f32, like the
+    // total = sum over experts in index order groups (one warp sum per 32-wide slice, slices added in order): f32, like the
     // reference's simd_sum per 32-wide slice accumulated over slices
+    float sum[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        pv[j] = valid[j] ? expf(pv[j] - max_logit) : 0.0f;
+        sum[j] = pv[j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < PER; ++j) sum[j] += __shfl_xor_sync(0xFFFFFFFFu, sum[j], o);
     float total = 0.0f;
 #pragma unroll
-    for (int j = 0; j < kMaxPer; ++j) {
-        if (j >= per) break;   // warp-uniform: slices beyond the expert count hold nothing
-        float ex = valid[j] ? expf(pv[j] - max_logit) : 0.0f;
-        pv[j] = ex;
-        float s = ex;
+    for (int j = 0; j < PER; ++j) total += sum[j];
+    // Valid weights are softmax outputs (finite, >= 0), so their bit patterns order like the values: key = bits + 1, 0 for an
+    // expert that cannot be chosen (any more).
+    uint32_t key[PER];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-        total += s;
-    }
-#pragma unroll
-    for (int j = 0; j < kMaxPer; ++j) {
-        valid[j] = valid[j] && total > 0.0f;
-        pv[j] = valid[j] ? pv[j] / total : -1e30f;
-    }
+    for (int j = 0; j < PER; ++j) key[j] = valid[j] && total > 0.0f ? __float_as_uint(pv[j] / total) + 1u : 0u;
     float sel_w = 0.0f;   // lane r keeps the weight of the r-th choice
     int sel_i = -1;
     float acc = 0.0f;
     for (int r = 0; r < k; ++r) {
-        float bv = -3.4e38f;
-        int bi = 0x7FFFFFFF;
+        uint32_t best = 0u;
+        int bj = 0;
 #pragma unroll
-        for (int j = 0; j < kMaxPer; ++j) {
-            if (j >= per) break;
-            const int id = lane + 32 * j;
-            if (valid[j] && (pv[j] > bv || (pv[j] == bv && id < bi))) {
-                bv = pv[j];
-                bi = id;
+        for (int j = 0; j < PER; ++j)
+            if (key[j] > best) {   // ties inside a lane go to the lower expert
+                best = key[j];
+                bj = j;
             }
-        }
-        // warp argmax with ties to the lower id.  Valid weights are softmax outputs (finite, >= 0), so their bit patterns
-        // order like the values: one integer max over the warp, then the lowest id among the lanes that hold it.
-        const uint32_t key = bi != 0x7FFFFFFF ? __float_as_uint(bv) + 1u : 0u;   // 0: this lane has no candidate
-        const uint32_t kmax = __reduce_max_sync(0xFFFFFFFFu, key);
-        const uint32_t cand = (kmax != 0u && key == kmax) ? static_cast<uint32_t>(bi) : 0x7FFFFFFFu;
-        bi = static_cast<int>(__reduce_min_sync(0xFFFFFFFFu, cand));
-        bv = kmax != 0u ? __uint_as_float(kmax - 1u) : -3.4e38f;
-        const bool found = bi != 0x7FFFFFFF;
-        if (found && (bi & 31) == lane) {
+        // warp argmax with ties to the lower id: one integer max over the warp, then the lowest id among the lanes that hold it
+        const uint32_t kmax = __reduce_max_sync(0xFFFFFFFFu, best);
+        const uint32_t cand = (kmax != 0u && best == kmax) ? static_cast<uint32_t>(lane + 32 * bj) : 0x7FFFFFFFu;
+        const int bi = static_cast<int>(__reduce_min_sync(0xFFFFFFFFu, cand));
+        const bool found = kmax != 0u;
+        const float bv = found ? __uint_as_float(kmax - 1u) : 0.0f;
 #pragma unroll
-            for (int j = 0; j < kMaxPer; ++j)
-                if (j == (bi >> 5)) valid[j] = false;
-        }
+        for (int j = 0; j < PER; ++j)
+            if (lane + 32 * j == bi) key[j] = 0u;
         if (lane == r) {
-            sel_w = found ? bv : 0.0f;
+            sel_w = bv;
             sel_i = found ? bi : -1;
         }
-        acc += found ? bv : 0.0f;   // same order on every lane: sum of the chosen weights in rank order
+        acc += bv;   // same order on every lane: sum of the chosen weights in rank order
     }
+    const float rs = routed_scale > 0.0f ? routed_scale : 1.0f;
+    const float nw = norm_topk ? (acc > 0.0f ? sel_w / acc : 0.0f) : sel_w;
+    out_i = sel_i;
+    out_w = nw * rs;
+}
+
+template <int PER>
+__global__ void __launch_bounds__(128) qwc_moe_route_kernel(const float* __restrict__ logits, int t_rows, int e, int k,
+                                                            int norm_topk, float routed_scale, int32_t* __restrict__ idx,
+                                                            float* __restrict__ wts) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31;
+    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (t >= t_rows) return;
+    int ci;
+    float cw;
+    moe_route_token<PER>(logits + static_cast<int64_t>(t) * e, e, k, norm_topk, routed_scale, lane, ci, cw);
     if (lane < k) {
-        const float rs = routed_scale > 0.0f ? routed_scale : 1.0f;
-        const float nw = norm_topk ? (acc > 0.0f ? sel_w / acc : 0.0f) : sel_w;
-        idx[static_cast<int64_t>(t) * k + lane] = sel_i;
-        wts[static_cast<int64_t>(t) * k + lane] = nw * rs;
+        idx[static_cast<int64_t>(t) * k + lane] = ci;
+        wts[static_cast<int64_t>(t) * k + lane] = cw;
     }
 }
 
@@ -423,44 +433,75 @@ __global__ void __launch_bounds__(kSortCta) qwc_moe_sort_kernel(const int32_t* _
     }
 }
 
-// Decode-time plan (at most 8 tokens, so an expert holds at most 8 sorted rows): one list entry per (active expert,
-// block of output columns) for the gate/up and for the down matmul, each entry served by one CTA of the streaming GEMV
-// in segment mode (the twin of the reference's per-(token, route) GEMVs with expert de-duplication,
+// Decode-time front (at most 8 tokens, so at most 128 pairs and at most 8 sorted rows per expert): routing, pair sort, list of
+// work and gather in one launch.  As four launches of a CTA or a few they were bound by their latencies (isolated 8.4 + 5.7 +
+// 3.7 + 3.5 us at 4 tokens, top-8 of 256 experts); the block, router included, went from 56.0 to 42.5 us.  Every CTA routes
+// all tokens (a warp each) and sorts all pairs in shared memory, which costs less than handing the result from one grid to
+// the next; then each gathers its share of the rows, and CTA 0 publishes the weights, the positions and the lists.
+// A list entry is one (active expert, block of output columns) of the gate/up or of the down matmul, served by one CTA of the
+// streaming GEMV in segment mode (the twin of the reference's per-(token, route) GEMVs with expert de-duplication,
 // Sources/Operators/QWGEMM/QWGemmMoE.swift:117-199).  Entry layout = qwc_gemv_seg of qwc_gemv.cu.
 struct MoeSeg {
     int32_t w_row0, col0, cols, x_row0, m, pad0, pad1, pad2;
 };
+constexpr int kFrontTokens = 8, kFrontPairs = kFrontTokens * 16;   // top-k <= 16
 
-__global__ void __launch_bounds__(512) qwc_moe_decode_plan_kernel(const int32_t* __restrict__ expert_off, int e, int inter, int h,
-                                                                  int cols_gu, int cols_dn, MoeSeg* __restrict__ segs_gu,
-                                                                  MoeSeg* __restrict__ segs_dn, int32_t* __restrict__ seg_counts) {
+template <int PER>
+__global__ void __launch_bounds__(32 * kFrontTokens)
+qwc_moe_decode_front_kernel(const float* __restrict__ logits, int t_rows, int e, int k, int norm_topk, float routed_scale,
+                            const __half* __restrict__ x, int64_t ldx, int h, int inter, int rotate, int vec, int cols_gu, int cols_dn,
+                            float* __restrict__ wts, int32_t* __restrict__ inv_perm, MoeSeg* __restrict__ segs_gu,
+                            MoeSeg* __restrict__ segs_dn, int32_t* __restrict__ seg_counts, __half* __restrict__ xs) {
+    __shared__ int s_idx[kFrontPairs];    // expert of a pair; kNone: dropped
+    __shared__ int s_first[kFrontPairs];  // the same for the first pair of an expert, kNone for the others
+    __shared__ int s_tok[kFrontPairs];    // token of a sorted row
+    constexpr int kNone = 0x7FFFFFFF;
     pdl_enter();
-    __shared__ int s_warp[16];
-    const int ex = threadIdx.x, lane = ex & 31, warp = ex >> 5;
-    const int cnt = ex < e ? expert_off[ex + 1] - expert_off[ex] : 0;
-    const unsigned act = __ballot_sync(0xFFFFFFFFu, cnt > 0);
-    if (lane == 0) s_warp[warp] = __popc(act);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int pairs = t_rows * k;
+    if (warp < t_rows) {
+        int ci;
+        float cw;
+        moe_route_token<PER>(logits + static_cast<int64_t>(warp) * e, e, k, norm_topk, routed_scale, lane, ci, cw);
+        if (lane < k) {
+            s_idx[warp * k + lane] = ci >= 0 ? ci : kNone;
+            if (blockIdx.x == 0) wts[warp * k + lane] = cw;
+        }
+    }
     __syncthreads();
-    int before = __popc(act & ((1u << lane) - 1u)), total = 0;
-    for (int w = 0; w < 16; ++w) {
-        if (w < warp) before += s_warp[w];
-        total += s_warp[w];
+    // Stable counting sort by comparison: a pair's position is the number of pairs of lower experts plus the earlier ones of its own.
+    const int v = tid < pairs ? s_idx[tid] : kNone;
+    int lower = 0, before = 0, same = 0;
+    if (v != kNone)
+        for (int q = 0; q < pairs; ++q) {
+            const int o = s_idx[q];
+            lower += o < v;
+            same += o == v;
+            before += o == v && q < tid;
+        }
+    const bool first = v != kNone && before == 0;
+    if (tid < pairs) s_first[tid] = first ? v : kNone;
+    if (v != kNone) s_tok[lower + before] = tid / k;
+    const int rows = __syncthreads_count(v != kNone);
+    if (blockIdx.x == 0) {
+        const int active = __syncthreads_count(first);
+        const int ngu = (inter + cols_gu - 1) / cols_gu, ndn = (h + cols_dn - 1) / cols_dn;
+        if (tid == 0) {
+            seg_counts[0] = active * ngu;
+            seg_counts[1] = active * ndn;
+        }
+        if (tid < pairs) inv_perm[tid] = v != kNone ? lower + before : -1;
+        if (first) {
+            int rank = 0;   // of this expert among the active ones
+            for (int q = 0; q < pairs; ++q) rank += s_first[q] < v;
+            for (int j = 0; j < ngu; ++j)
+                segs_gu[rank * ngu + j] = MoeSeg{v * 2 * inter, j * cols_gu, min(cols_gu, inter - j * cols_gu), lower, same, 0, 0, 0};
+            for (int j = 0; j < ndn; ++j)
+                segs_dn[rank * ndn + j] = MoeSeg{v * h, j * cols_dn, min(cols_dn, h - j * cols_dn), lower, same, 0, 0, 0};
+        }
     }
-    const int ngu = (inter + cols_gu - 1) / cols_gu, ndn = (h + cols_dn - 1) / cols_dn;
-    if (ex == 0) {
-        seg_counts[0] = total * ngu;
-        seg_counts[1] = total * ndn;
-    }
-    if (cnt <= 0) return;
-    const int x0 = expert_off[ex];
-    for (int j = 0; j < ngu; ++j) {
-        MoeSeg sg{ex * 2 * inter, j * cols_gu, min(cols_gu, inter - j * cols_gu), x0, min(cnt, 8), 0, 0, 0};
-        segs_gu[before * ngu + j] = sg;
-    }
-    for (int j = 0; j < ndn; ++j) {
-        MoeSeg sg{ex * h, j * cols_dn, min(cols_dn, h - j * cols_dn), x0, min(cnt, 8), 0, 0, 0};
-        segs_dn[before * ndn + j] = sg;
-    }
+    moe_gather_items<uint32_t>(x, ldx, h, s_tok, static_cast<uint32_t>(rows), rotate, vec, xs, static_cast<int>(blockIdx.x),
+                               static_cast<int>(gridDim.x));
 }
 
 // xs[p, :] = xr[sorted_tok[p], :] for rows that are rotated already: one warp per sorted row, 16 bytes per lane and step, four
@@ -609,6 +650,9 @@ int grid_for(const qwc_hal* hal, int64_t items, int per_block, int waves) {
     return static_cast<int>(g);
 }
 
+// The routing kernels' instantiation for e <= 512 experts: 4, 8 or 16 slices of 32.
+template <typename Fn> Fn moe_by_slices(int64_t e, Fn s4, Fn s8, Fn s16) { return e <= 128 ? s4 : (e <= 256 ? s8 : s16); }
+
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Scratch layout of qwc_moe_forward (every region 256-byte aligned).
@@ -667,8 +711,9 @@ int qwc_moe_route(qwc_hal* hal, qwc_stream stream, const float* logits, int64_t 
     if (t == 0) return QWC_OK;
     if (!logits || !idx || !wts) return qwc_fail(QWC_ERR_BAD_SHAPE, "null buffer");
     const int blocks = static_cast<int>((t + 3) / 4);
-    QWC_CUDA_TRY(qwc_launch_pdl(qwc_moe_route_kernel, dim3(blocks), dim3(128), 0, static_cast<cudaStream_t>(stream), logits,
-                                static_cast<int>(t), static_cast<int>(e), static_cast<int>(k), norm_topk, routed_scale, idx, wts));
+    const auto kernel = moe_by_slices(e, qwc_moe_route_kernel<4>, qwc_moe_route_kernel<8>, qwc_moe_route_kernel<16>);
+    QWC_CUDA_TRY(qwc_launch_pdl(kernel, dim3(blocks), dim3(128), 0, static_cast<cudaStream_t>(stream), logits, static_cast<int>(t),
+                                static_cast<int>(e), static_cast<int>(k), norm_topk, routed_scale, idx, wts));
     return QWC_OK;
 }
 
@@ -943,22 +988,24 @@ int qwc_moe_forward(qwc_hal* hal, qwc_stream stream, const qwc_weight_view* bank
     if (!decode_path && (!qwc_gemm_tc_supported(hal, bank_gu, 17, QWC_EPI_NONE) || !qwc_gemm_tc_supported(hal, bank_dn, 17, QWC_EPI_NONE)))
         return qwc_fail(QWC_ERR_BLOCKED, "the grouped expert GEMMs need HQ4_G32_M5 / HQ8_G32 banks with k %% 128 == 0 or HQ4_G64 banks with k %% 256 == 0, "
                                          "16-byte aligned");
-    if ((rc = qwc_moe_route(hal, stream, logits, t, e, k, norm_topk, routed_scale, idx, wts))) return rc;
     if (decode_path) {
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        if ((rc = qwc_moe_group_pairs(hal, stream, idx, pairs, e, k, expert_off, sorted_pair, sorted_tok, inv_perm, 2 * inter, h,
-                                      QWC_EPI_NONE, nullptr, nullptr, tile_counts))) return rc;
         MoeSeg* segs_gu = reinterpret_cast<MoeSeg*>(tiles_gu);
         MoeSeg* segs_dn = reinterpret_cast<MoeSeg*>(tiles_dn);
-        QWC_CUDA_TRY(qwc_launch_pdl(qwc_moe_decode_plan_kernel, dim3(1), dim3(512), 0, st, expert_off, static_cast<int>(e),
-                                    static_cast<int>(inter), static_cast<int>(h), cols_gu, cols_dn, segs_gu, segs_dn, tile_counts + 2));
-        if ((rc = qwc_moe_gather(hal, stream, x_f16, ldx, h, sorted_tok, expert_off, e, pairs, x_is_rotated, sc + L.xs))) return rc;
+        const auto front = moe_by_slices(e, qwc_moe_decode_front_kernel<4>, qwc_moe_decode_front_kernel<8>, qwc_moe_decode_front_kernel<16>);
+        const int vec = reinterpret_cast<uintptr_t>(x_f16) % 16 == 0 && ldx % 8 == 0;
+        QWC_CUDA_TRY(qwc_launch_pdl(front, dim3(grid_for(hal, pairs * (h / 32), 64, 1)), dim3(32 * kFrontTokens), 0, st, logits,
+                                    static_cast<int>(t), static_cast<int>(e), static_cast<int>(k), static_cast<int>(norm_topk), routed_scale,
+                                    static_cast<const __half*>(x_f16), ldx, static_cast<int>(h), static_cast<int>(inter),
+                                    static_cast<int>(!x_is_rotated), vec, cols_gu, cols_dn, wts, inv_perm, segs_gu, segs_dn,
+                                    tile_counts + 2, reinterpret_cast<__half*>(sc + L.xs)));
         if ((rc = qwc_launch_gemv_segments(hal, st, bank_gu, sc + L.xs, h, sc + L.hs, QWC_F16, inter, QWC_EPI_SILU_PAIR_FWHT, inter,
                                            cols_gu, segs_gu, tile_counts + 2, max_gu))) return rc;
         if ((rc = qwc_launch_gemv_segments(hal, st, bank_dn, sc + L.hs, inter, sc + L.dn, QWC_F16, h, QWC_EPI_NONE, h, cols_dn,
                                            segs_dn, tile_counts + 3, max_dn))) return rc;
         return qwc_moe_combine(hal, stream, sc + L.dn, QWC_F16, inv_perm, wts, t, k, h, out, out_dtype);
     }
+    if ((rc = qwc_moe_route(hal, stream, logits, t, e, k, norm_topk, routed_scale, idx, wts))) return rc;
     // SwiGLU + FWHT run in the gate/up GEMM's epilogue when the tiles can pair 64 gate rows with their up rows
     const int32_t gu_epi = inter % 64 == 0 ? QWC_EPI_SILU_PAIR_FWHT : QWC_EPI_NONE;
     // The gate/up region of the scratch is idle until the gate/up GEMM writes it (never, with the fused epilogue): it holds the

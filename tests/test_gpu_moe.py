@@ -147,6 +147,51 @@ def test_moe_forward_vs_oracle(hal, oracle, cfg, name):
     assert_matmul_close(out16.float().cpu().numpy(), ref, tight=8e-3)
 
 
+# The one-launch decode front (routing, sort, list and gather for at most 8 tokens): both ends of tokens, experts and top-k,
+# expert counts around its 32-wide slices and instantiations (128, 256), tokens without a finite logit (all routes dropped),
+# rows that are not 16-byte aligned, rotated rows.  Static-weights mode, two routings back to back on one scratch, so that a
+# kernel that read the other call's list would show.
+@pytest.mark.parametrize("t,e,k,hidden,inter", [(1, 1, 1, 128, 128), (8, 16, 16, 128, 256), (3, 33, 2, 256, 128), (8, 129, 16, 128, 128),
+                                                (7, 257, 5, 128, 128), (2, 512, 16, 128, 128), (8, 128, 1, 1024, 128)])
+@pytest.mark.parametrize("rotated", [False, True])
+def test_moe_decode_front_edges(hal, oracle, t, e, k, hidden, inter, rotated):
+    import qwegn_b200 as q
+    fmt, cont = oracle.FORMATS["HQ4_G32"], q.CONTAINERS["HQ4_G32"]
+    rng = np.random.default_rng(t * 1000 + e)
+    gu, dn = _expert_banks(oracle, fmt, e, hidden, inter, rng)
+    bank_gu = q.QWWeightView(torch.from_numpy(gu.reshape(-1)).cuda(), e * 2 * inter, hidden, cont)
+    bank_dn = q.QWWeightView(torch.from_numpy(dn.reshape(-1)).cuda(), e * hidden, inter, cont)
+    op = q.QWMoEOperator(hal, bank_gu, bank_dn, e, inter, k, norm_topk=True)
+    scratch = torch.empty(op.scratchBytes(t), dtype=torch.uint8, device="cuda")
+    calls = []
+    for shift in (0, 1):
+        x = rng.standard_normal((t, hidden)).astype(np.float16)
+        lg = rng.standard_normal((t, e)).astype(np.float32)
+        if t > 1:
+            lg[t - 1] = np.nan
+            lg[0, 0] = np.inf
+        xd = torch.empty(t * (hidden + shift), dtype=torch.float16, device="cuda").view(t, hidden + shift)[:, :hidden]
+        xd.copy_(torch.from_numpy(oracle.fwht32_f16(x) if rotated else x))
+        ridx, rwts = oracle.moe_route(lg, k, norm_topk=True)
+        calls.append((xd, torch.from_numpy(lg).cuda(), torch.full((t, hidden), float("nan"), device="cuda"),
+                      oracle.moe_forward(gu, dn, fmt, e, hidden, inter, x, ridx, rwts)))
+    torch.cuda.synchronize()
+    hal.set_static_weights(True)
+    try:
+        for _ in range(3):
+            for xd, lg, out, _ref in calls:
+                op.encodeResident(xd, lg, out, scratch, x_is_rotated=rotated)
+        torch.cuda.synchronize()
+    finally:
+        hal.set_static_weights(False)
+    for _x, _lg, out, ref in calls:
+        got = out.cpu().numpy()
+        assert np.isfinite(got).all()
+        if t > 1:
+            assert not got[t - 1].any()
+        assert_matmul_close(got, ref, tight=6e-3)
+
+
 @pytest.mark.parametrize("name", ["HQ4_G32", "HQ8_G32"])
 def test_gate_up_doors_fused_and_unfused_agree(hal, oracle, name):
     # Door by door: pair sort -> gather -> grouped gate/up GEMM -> SwiGLU + FWHT as its own kernel, against the same
