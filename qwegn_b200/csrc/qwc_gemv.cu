@@ -96,6 +96,7 @@ struct GemvParams {
     // segment mode (see the kernel): null in the ordinary one-bank form
     const qwc_gemv_seg* segs;
     const int32_t* seg_count;
+    int segs_done;            // the list is complete when this grid may start (see the kernel)
     int seg_grid, seg_cols;   // host side: capacity of the list (= grid) and output columns per entry
     // fused one-shot all-reduce over peer memory (row-parallel shards of a tensor-parallel group; ar_world > 1):
     int ar_world, ar_rank;
@@ -234,9 +235,15 @@ qwc_gemv_stream_kernel(const GemvParams p, const __grid_constant__ CUtensorMap t
     using C = StreamCfg<FMT>;
     if (p.segs != nullptr) {
         // The segment list is the work of a kernel earlier in the stream: a programmatic launch must wait for it
-        // before the first read (nothing can be prefetched without the list anyway).
-        if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (static_cast<int>(blockIdx.x) >= *p.seg_count) return;   // whole CTA: nothing is set up yet
+        // before the first read (nothing can be prefetched without the list anyway) -- unless the launch before this one
+        // is the segment launch of the same call (segs_done).  That one waits here for the list's kernel, and only then
+        // lets this grid start (launch_dependents below): the list is complete and in memory, and this grid's weights can
+        // stream while the other's last CTAs finish (4 tokens, 256 experts top-8: 42.5 -> 41.2 us).  Read past L1.
+        if (p.pdl && !p.segs_done) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (static_cast<int>(blockIdx.x) >= __ldcg(p.seg_count)) {   // whole CTA: nothing is set up yet
+            if (p.pdl && p.segs_done) asm volatile("griddepcontrol.wait;" ::: "memory");   // this grid ends after the one before it
+            return;
+        }
     }
     extern __shared__ __align__(128) uint8_t smem[];
     // layout: [x region][reduction region][barriers][stages...]
@@ -281,7 +288,8 @@ qwc_gemv_stream_kernel(const GemvParams p, const __grid_constant__ CUtensorMap t
     void* Y_ = p.y;
     int64_t wbase = 0;   // weight row of output column 0
     if (p.segs != nullptr) {
-        const qwc_gemv_seg sg = p.segs[bq];   // the host launches exactly *seg_count CTAs' worth or more; extra CTAs left above
+        const int4 s0 = __ldcg(reinterpret_cast<const int4*>(p.segs + bq));
+        const qwc_gemv_seg sg{s0.x, s0.y, s0.z, s0.w, __ldcg(&p.segs[bq].m), 0, 0, 0};   // the host launches exactly *seg_count CTAs' worth or more; extra CTAs left above
         rb = sg.col0;
         re = sg.col0 + sg.cols;
         M_ = sg.m;
@@ -1163,9 +1171,10 @@ int qwc_launch_gemv_ar(const qwc_hal* hal, cudaStream_t st, const qwc_weight_vie
 // Segment mode of the stream kernel (decode-time mixture of experts): `bank` is the stacked expert bank, xs the
 // expert-sorted (rotated) activation rows, y the expert-sorted outputs [pairs, n_out]; entry i of the device-side list
 // `segs` (at most max_segs entries, *seg_count valid) names one expert's column range and its <= 8 rows.
+// after_segments: the launch before this one in the stream is a segment launch that waited for the kernel that made this list.
 int qwc_launch_gemv_segments(const qwc_hal* hal, cudaStream_t st, const qwc_weight_view* bank, const void* xs, int64_t ldx,
                              void* y, int y_dtype, int64_t ldy, int epilogue, int64_t n_out, int seg_cols, const void* segs,
-                             const int32_t* seg_count, int64_t max_segs) {
+                             const int32_t* seg_count, int64_t max_segs, bool after_segments) {
     GemvParams p{};
     const int fmt = qwc_fmt_of(*bank);
     const int64_t bb = qwc_block_bytes(bank->kind, bank->bits, bank->group);
@@ -1187,6 +1196,7 @@ int qwc_launch_gemv_segments(const qwc_hal* hal, cudaStream_t st, const qwc_weig
     p.pdl = hal->static_weights;
     p.segs = static_cast<const qwc_gemv_seg*>(segs);
     p.seg_count = seg_count;
+    p.segs_done = after_segments;
     p.seg_grid = static_cast<int>(max_segs);
     p.seg_cols = seg_cols;
     if (p.row_bytes % 16 != 0 || reinterpret_cast<uintptr_t>(bank->blocks) % 16 != 0)

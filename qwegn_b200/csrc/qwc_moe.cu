@@ -14,7 +14,7 @@ int qwc_launch_gemm_tc_grouped(const qwc_hal*, cudaStream_t, const qwc_weight_vi
                                const int32_t*, int64_t, void*, int, int64_t, int, int, int);
 bool qwc_gemm_tc_supported(const qwc_hal*, const qwc_weight_view*, int64_t, int);
 int qwc_launch_gemv_segments(const qwc_hal*, cudaStream_t, const qwc_weight_view*, const void*, int64_t, void*, int, int64_t, int,
-                             int64_t, int, const void*, const int32_t*, int64_t);
+                             int64_t, int, const void*, const int32_t*, int64_t, bool);
 
 namespace {
 
@@ -1000,9 +1000,9 @@ int qwc_moe_forward(qwc_hal* hal, qwc_stream stream, const qwc_weight_view* bank
                                     static_cast<int>(!x_is_rotated), vec, cols_gu, cols_dn, wts, inv_perm, segs_gu, segs_dn,
                                     tile_counts + 2, reinterpret_cast<__half*>(sc + L.xs)));
         if ((rc = qwc_launch_gemv_segments(hal, st, bank_gu, sc + L.xs, h, sc + L.hs, QWC_F16, inter, QWC_EPI_SILU_PAIR_FWHT, inter,
-                                           cols_gu, segs_gu, tile_counts + 2, max_gu))) return rc;
+                                           cols_gu, segs_gu, tile_counts + 2, max_gu, false))) return rc;
         if ((rc = qwc_launch_gemv_segments(hal, st, bank_dn, sc + L.hs, inter, sc + L.dn, QWC_F16, h, QWC_EPI_NONE, h, cols_dn,
-                                           segs_dn, tile_counts + 3, max_dn))) return rc;
+                                           segs_dn, tile_counts + 3, max_dn, true))) return rc;
         return qwc_moe_combine(hal, stream, sc + L.dn, QWC_F16, inv_perm, wts, t, k, h, out, out_dtype);
     }
     if ((rc = qwc_moe_route(hal, stream, logits, t, e, k, norm_topk, routed_scale, idx, wts))) return rc;
