@@ -11,10 +11,15 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-// One CTA per row; thread t owns the 16-byte chunks t, t + T, ... (8 halves each).  A quad of consecutive threads
-// holds one aligned 32-element block, so the FWHT-32 is three in-lane butterfly stages plus two xor-shuffle stages.
+// One CTA per row; thread t owns the 16-byte chunks t, t + T, ... (8 halves each), CH of them at most.  A quad of consecutive
+// threads holds one aligned 32-element block, so the FWHT-32 is three in-lane butterfly stages plus two xor-shuffle stages.
+// A row is a chain of latencies (load, sum over the CTA, store): as many threads as chunks, and gamma is loaded with the
+// row instead of behind the sum.  CH is a template argument because registers for four chunks left room for one CTA of
+// 640 threads on an SM; with one chunk three fit.  Before / now, us, with residual: 1 x 5120 2.34 / 2.05, 333 x 5120 3.88 /
+// 3.65, 4096 x 5120 31.8 / 26.9, 4096 x 8192 50.4 / 41.2 (168 and 268 MB: 26 and 42 us at 6.46 TB/s).
 constexpr int kNormMaxChunks = 4;   // chunks kept in registers per thread (hidden <= 8 * 4 * blockDim)
 
+template <int CH>
 __global__ void __launch_bounds__(1024) qwc_rmsnorm_fwht_kernel(const __half* __restrict__ x, const __half* __restrict__ gamma,
                                                                 __half* __restrict__ y, __half* residual, int hidden, float eps,
                                                                 int rotate) {
@@ -29,29 +34,34 @@ __global__ void __launch_bounds__(1024) qwc_rmsnorm_fwht_kernel(const __half* __
     uint4* yr = reinterpret_cast<uint4*>(y + row * hidden);
     const uint4* gr = reinterpret_cast<const uint4*>(gamma);
 
-    uint4 reg[kNormMaxChunks];
+    uint4 reg[CH], res[CH], gam[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+        if (tid + i * nthreads < chunks) {
+            reg[i] = xr[tid + i * nthreads];
+            if (rr) res[i] = rr[tid + i * nthreads];
+        }
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+        if (tid + i * nthreads < chunks) gam[i] = gr[tid + i * nthreads];
     float acc = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kNormMaxChunks; ++i) {
+    for (int i = 0; i < CH; ++i) {
         const int u = tid + i * nthreads;
         if (u < chunks) {
-            uint4 v = xr[u];
+            __half2* a = reinterpret_cast<__half2*>(&reg[i]);
             if (rr) {
-                const uint4 r = rr[u];
-                __half2* a = reinterpret_cast<__half2*>(&v);
-                const __half2* b = reinterpret_cast<const __half2*>(&r);
+                const __half2* b = reinterpret_cast<const __half2*>(&res[i]);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 fa = __half22float2(a[j]), fb = __half22float2(b[j]);
                     a[j] = __floats2half2_rn(__fadd_rn(fa.x, fb.x), __fadd_rn(fa.y, fb.y));
                 }
-                rr[u] = v;   // residual += x, kept in f16 as the reference does
+                rr[u] = reg[i];   // residual += x, kept in f16 as the reference does
             }
-            reg[i] = v;
-            const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float2 f = __half22float2(h[j]);
+                const float2 f = __half22float2(a[j]);
                 acc = fmaf(f.x, f.x, acc);
                 acc = fmaf(f.y, f.y, acc);
             }
@@ -71,12 +81,11 @@ __global__ void __launch_bounds__(1024) qwc_rmsnorm_fwht_kernel(const __half* __
     const float rstd = s_rstd;
     const int t4 = lane & 3;
 #pragma unroll
-    for (int i = 0; i < kNormMaxChunks; ++i) {
+    for (int i = 0; i < CH; ++i) {
         const int u = tid + i * nthreads;
         if (u < chunks) {   // uniform per warp: chunks and nthreads are multiples of 32
-            const uint4 g = gr[u];
             const __half2* h = reinterpret_cast<const __half2*>(&reg[i]);
-            const __half2* gh = reinterpret_cast<const __half2*>(&g);
+            const __half2* gh = reinterpret_cast<const __half2*>(&gam[i]);
             float f[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -250,7 +259,12 @@ extern "C" int qwc_rmsnorm_fwht(qwc_hal* hal, qwc_stream stream, const void* x_f
     if (threads < 32) threads = 32;
     // more threads than strictly needed (up to one chunk per thread) shorten a row's latency at decode
     while (threads * 2 <= chunks && threads * 2 <= 1024) threads *= 2;
-    QWC_CUDA_TRY(qwc_launch_pdl(qwc_rmsnorm_fwht_kernel, dim3(static_cast<unsigned>(rows)), dim3(threads), 0, static_cast<cudaStream_t>(stream),
+    // Rows beyond one wave of such CTAs: two chunks per thread keep more bytes in flight (4096 x 5120 30.5 -> 26.9 us, 1024 x 8192
+    // 15.2 -> 12.6; within one wave they only lengthen the row's chain, 333 x 5120 3.65 -> 4.15 us).
+    if (threads == chunks && threads % 64 == 0 && rows > static_cast<int64_t>(hal->sm_count) * (2048 / threads)) threads /= 2;
+    const int per = (chunks + threads - 1) / threads;
+    const auto kernel = per == 1 ? qwc_rmsnorm_fwht_kernel<1> : (per == 2 ? qwc_rmsnorm_fwht_kernel<2> : qwc_rmsnorm_fwht_kernel<kNormMaxChunks>);
+    QWC_CUDA_TRY(qwc_launch_pdl(kernel, dim3(static_cast<unsigned>(rows)), dim3(threads), 0, static_cast<cudaStream_t>(stream),
                                 static_cast<const __half*>(x_f16), static_cast<const __half*>(gamma_f16), static_cast<__half*>(y_f16),
                                 static_cast<__half*>(residual_f16), static_cast<int>(hidden), eps, rotate));
     return QWC_OK;

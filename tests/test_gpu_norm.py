@@ -30,6 +30,13 @@ def test_rmsnorm_fwht_matches_the_oracle(hal, oracle, rows, hidden, with_residua
         assert np.array_equal(rd.cpu().numpy(), rref)   # residual += x, rounded to f16 once
 
 
+# The block sizes of the norm: the most rows of one wave of one-chunk CTAs and one row more (148 SMs x 2048 / threads), the
+# smallest row, rows of two and of four chunks per thread.
+@pytest.mark.parametrize("rows,hidden", [(1184, 2048), (1185, 2048), (445, 5120), (297, 8192), (9473, 256), (3, 16384), (2, 32768), (1, 768)])
+def test_rmsnorm_block_shapes(hal, oracle, rows, hidden):
+    test_rmsnorm_fwht_matches_the_oracle(hal, oracle, rows, hidden, True, True)
+
+
 def test_rmsnorm_feeds_the_matmul(hal, oracle):
     # norm -> GEMV with x_is_rotated=1 equals GEMV on the un-rotated normalised activations
     import qwegn_b200 as q
