@@ -144,17 +144,6 @@ __device__ __forceinline__ void router_mma(float d[4], uint32_t a0, uint32_t a1,
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ void router_mma_tf32(float d[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// Element HI of a pair as f32 bits (exact in tf32: f16 has as many significant bits, bf16 fewer; f16 subnormals become normal).
-template <int HI> __device__ __forceinline__ uint32_t pair_f32(uint32_t v, const __half*) {
-    const __half2 h = *reinterpret_cast<const __half2*>(&v);
-    return __float_as_uint(HI ? __high2float(h) : __low2float(h));
-}
-template <int HI> __device__ __forceinline__ uint32_t pair_f32(uint32_t v, const unsigned short*) { return HI ? v & 0xFFFF0000u : v << 16; }
-
 template <int RAW, typename T> __device__ __forceinline__ void load_raw(const T* p, uint32_t* r) {
     const uint4 a = *reinterpret_cast<const uint4*>(p);
     r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
@@ -173,10 +162,6 @@ template <typename XT, typename WT, int MW, int NW, int KW>
 __global__ void __launch_bounds__(MW * NW * KW * 32, 1) qwc_router_mma_kernel(const XT* __restrict__ x, int64_t ldx, const WT* __restrict__ w,
                                                                              int t_rows, int e, int h, float* __restrict__ y) {
     constexpr bool kF16 = sizeof(XT) == 2 && RouterPlanes<WT>::kPlanes == 2;   // x f16 (2-byte x is always f16), w f16
-    // x f16 with w bf16: both are exact in tf32, so one pass of k8 MMAs takes them as they are.  It is as many tensor cycles as the
-    // two planes of x in bf16, but two instructions per pair of elements instead of about ten to make the operands.  2048
-    // tokens, 256 experts top-8: block 299.3 -> 296.3 us.
-    constexpr bool kTf32 = sizeof(XT) == 2 && sizeof(WT) == 2 && !kF16;
     constexpr int PX = kF16 ? 1 : RouterPlanes<XT>::kPlanes, PW = kF16 ? 1 : RouterPlanes<WT>::kPlanes;
     constexpr int RX = RouterPlanes<XT>::kRaw, RW = RouterPlanes<WT>::kRaw;
     constexpr int TM = 32 * MW, TN = 32 * NW;
@@ -210,36 +195,6 @@ __global__ void __launch_bounds__(MW * NW * KW * 32, 1) qwc_router_mma_kernel(co
         }
     }
     for (int s = kw; s < steps; s += KW) {
-        if constexpr (kTf32) {
-            uint32_t xc[4][4], wc[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) { xc[i][j] = xr[i][j]; wc[i][j] = wr[i][j]; }
-            if (s + KW < steps) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    load_raw<RX>(xp[i] + (s + KW) * 32, xr[i]);
-                    load_raw<RW>(wp[i] + (s + KW) * 32, wr[i]);
-                }
-            }
-            constexpr const XT* xt = nullptr;
-            constexpr const WT* wt = nullptr;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {   // k slots t4 and t4 + 4 of MMA q: elements 2 q and 2 q + 1 of the lane's eight
-                uint32_t b[4][2];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) { b[j][0] = pair_f32<0>(wc[j][q], wt); b[j][1] = pair_f32<1>(wc[j][q], wt); }
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint32_t a0 = pair_f32<0>(xc[2 * i][q], xt), a1 = pair_f32<0>(xc[2 * i + 1][q], xt);
-                    const uint32_t a2 = pair_f32<1>(xc[2 * i][q], xt), a3 = pair_f32<1>(xc[2 * i + 1][q], xt);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) router_mma_tf32(d[i][j], a0, a1, a2, a3, b[j][0], b[j][1]);
-                }
-            }
-            continue;
-        }
         uint32_t xpl[4][PX][4], wpl[4][PW][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
