@@ -75,6 +75,22 @@ def test_router_gemm_edges(hal, oracle, t, e, h, shift, xdt, wdt):
     assert (got[t] == 7.0).all()      # nothing is written past the last token
 
 
+# The error of a long K against 64 bits.  A sum of k products rounded to nearest at each of its additions is off by about
+# 2^-24 sqrt(k) of its size in the 2-norm when the sums are as large as the result; the split planes drop products below 2^-24.
+@pytest.mark.parametrize("xdt", [torch.float16, torch.float32])
+@pytest.mark.parametrize("wdt", [torch.bfloat16, torch.float16, torch.float32])
+def test_router_gemm_error_of_a_long_k(hal, xdt, wdt):
+    import qwegn_b200 as q
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    t, e, h = 70, 64, 7168
+    x = torch.randn(t, h, generator=gen, device="cuda").to(xdt)
+    w = (torch.randn(e, h, generator=gen, device="cuda") * h ** -0.5).to(wdt)
+    y = torch.empty(t, e, device="cuda")
+    q.QWGemmMoE.encodeFnRouterGemm(hal, w, x, y)
+    ref = x.double() @ w.double().T
+    assert float((y - ref).norm() / ref.norm()) < 2.0 ** -24 * (h / 32) ** 0.5   # h / 32 rounded additions: one per step of K
+
+
 def test_route_refusals(hal):
     import qwegn_b200 as q
     lg = torch.zeros((2, 600), dtype=torch.float32, device="cuda")
