@@ -8,9 +8,8 @@
 // One persistent CTA per SM walks (weight tile, token tile) pairs.  Roles: warp 0 activation TMA, warp 1 MMA issue
 // (+ TMEM allocation), warp 2 packed-weight TMA, 16 converter warps, 4 epilogue warps.
 //   * Per raw step a TMA copy brings 128 packed weight rows, unchanged, into a shared-memory ring (2-D tensor copy;
-//     one raw step = 128 k for the 20- and 36-byte blocks of 32, 256 k for the 36-byte blocks of 64, so that a row of a
-//     step is a multiple of 16 bytes); per 64-wide K tile another TMA copy brings the rotated activations (128-byte
-//     swizzle).
+//     one raw step = 512 k, 256 k of 8-bit codes; see TcFmt); per 64-wide K tile another TMA copy brings the rotated
+//     activations (128-byte swizzle).
 //   * A converter thread owns one weight row = one TMEM lane: it reads its row's 64 k of the raw step, decodes them in
 //     registers (magic-bias form and one f16 FMA with scale and bias: the reference's in-register decode,
 //     qw_gemm_nax.metalh:114-127) and only then waits for the operand stage to be free and writes 32 TMEM columns
@@ -20,11 +19,12 @@
 //     N = tokens, K = 16, into a TMEM accumulator; tcgen05.commit releases the stage and, after the last K tile, hands
 //     the accumulator to the epilogue warps (tcgen05.ld, lane = weight row; plain store or the fused SwiGLU (+ FWHT)
 //     epilogue); two accumulators alternate so the epilogue of one tile overlaps the main loop of the next.
-//   * TMEM budget (512 columns), four operand stages: tiles of up to 192 tokens use two 192-column accumulators and stages
-//     of one 64-wide K tile (32 columns of A each); tiles of up to 128 tokens (expert tiles, verify-sized calls) use two
-//     128-column accumulators and stages of two K tiles (64 columns of A, two activation sub-tiles), because the MMA
-//     warp's issue loop costs a fixed ~400 cycles per stage (barrier wait, fence, election, commit: measured with every
-//     other role idle) and with few tokens the MMAs of one K tile are shorter than that.
+//   * TMEM budget (512 columns): tiles of up to 192 tokens use two 192-column accumulators and operand stages of two 64-wide K
+//     tiles (64 columns of A each), tiles of up to 128 tokens (expert tiles, verify-sized calls) two 128-column accumulators
+//     and stages of four (128 columns), because the MMA warp's issue loop costs a fixed ~400 cycles per stage (barrier wait,
+//     fence, election, commit: measured with every other role idle) and with few tokens the MMAs of a K tile are shorter.
+//   * CTA pairs (CG = 2) share an activation tile: two weight tiles, one MMA of 256 rows, each CTA copies half of the
+//     activations.  A cluster may also split K of one tile when there are few tiles (partial sums meet in shared memory).
 // Weights are the M operand so that all tokens of a tile share every decoded weight.  The grouped (mixture-of-experts)
 // door runs the same kernel over a device-side tile list.  The kernel is launched with programmatic stream
 // serialization and waits for the grid before it (griddepcontrol.wait) after its own set-up, before any global access.
@@ -72,7 +72,7 @@ struct TcParams {
     int raw_stages;
     int a_stages;        // stages of decoded weights
     int x_stages;        // activation stages
-    int kt_per_stage;    // 64-wide K tiles per operand stage: 1 or 2 (a divisor of the K tiles of a raw step)
+    int kt_per_stage;    // 64-wide K tiles per operand stage: 2 or 4 (a divisor of the K tiles of a raw step)
     int acc_stride;      // TMEM columns per accumulator: 192 or 128; the operand stages start at column 2 * acc_stride
     int x_tile_rows;     // activation rows per tile: 192, 128 or 64
     int x_box[kXBoxes];  // rows of the activation boxes, tallest first
